@@ -13,10 +13,13 @@
 // produces block i's lower/upper envelope at frame i*aggStride, exactly when the
 // subtraction of that block starts, so the trace is read from HBM once and the
 // baselined trace written once, with coalesced 128-byte warp accesses.  The
-// window arrays of stages up to 11 wide live in shared memory, wider ones in
-// global memory, which leaves room for 14 one-lane blocks per SM (measured:
-// 3.45 ms a 1M-ZMW chunk against 4.10 ms with 17-wide windows in shared
-// memory at 12 blocks, 8.4 ms with every window in global memory).
+// windows of the scales that run every frame or every other frame live in
+// shared memory, those of the last scale (every 16 frames) in global memory,
+// which leaves room for 14 one-lane blocks per SM with the widest filter.
+// Bound by latency (a warp's dependent instructions; 3.5 warps a scheduler,
+// 48% of its issue slots).  4096 lanes x 512 frames of int16: 988 us with four
+// separate window stages a scale, conversions by I2F and F2I and selects in
+// the moments; 455 us as written (0.93 GB read and written, 2.0 TB/s).
 // Each stage window keeps the reference's van Herk/Gil-Werman state (ring of w
 // values, holdover, counter) so the filter outputs are bit-identical.
 #include <type_traits>
@@ -37,29 +40,50 @@ template <int FT> struct FLayout
 {
     using S = FSpec<FT>;
     static constexpr int nStages = 2 * S::n;           // per filter
-    static constexpr int kSmemMaxWidth = 11;           // wider windows stay in global memory (L1/L2)
     static constexpr int Width(int k) { return S::w[k / 2]; }
     // lower: erode, dilate, then erode/dilate; upper: dilate, erode, then erode/dilate
     static constexpr bool IsMax(bool upper, int k) { return (k < 2 && upper) ? (k == 0) : (k % 2 == 1); }
-    static constexpr bool InSmem(int k) { return Width(k) <= kSmemMaxWidth; }
+    static constexpr bool InSmem(int k) { return CumStride(k / 2) < AggStride(); }
     static constexpr int Idx(bool upper, int k) { return (upper ? nStages : 0) + k; }   // 0 .. 2*nStages-1
-    // Every stage keeps S[W] (suffix extrema of the previous block) and B[W]
-    // (inputs of the current block) in shared or global memory.
-    static constexpr int SmemSlots()
+    // Saved state: every stage's S[W] (suffix extrema of the previous block)
+    // and then its B[W] (inputs of the current block), first the stages up to
+    // 11 wide, then the wider ones, each group lower filter first.  (A state
+    // saved by one build is read by another: the order stays whatever the
+    // kernel keeps where.)
+    static constexpr bool Narrow(int k) { return Width(k) <= 11; }
+    static constexpr int SlotWindow(bool upper, int k)
     {
         int t = 0;
-        for (int k = 0; k < nStages; ++k) if (InSmem(k)) t += 2 * Width(k);
-        return 2 * t;
-    }
-    static constexpr int Offset(bool upper, int k)   // within its storage (smem or global)
-    {
-        int t = 0;
+        if (!Narrow(k))
+            for (int j = 0; j < nStages; ++j) if (Narrow(j)) t += 4 * Width(j);
         for (int u = 0; u < 2; ++u)
             for (int j = 0; j < nStages; ++j)
             {
                 if (u == (upper ? 1 : 0) && j == k) return t;
-                if (InSmem(j) == InSmem(k)) t += 2 * Width(j);
+                if (Narrow(j) == Narrow(k)) t += 2 * Width(j);
             }
+        return t;
+    }
+    // Shared memory: position c of a block needs S[c..] and B[..c-1] only, so
+    // a stage keeps one array of W there, inputs below the counter and suffix
+    // extrema from it on.
+    static constexpr int SmemSlots()
+    {
+        int t = 0;
+        for (int k = 0; k < nStages; ++k) if (InSmem(k)) t += 2 * Width(k);
+        return t;
+    }
+    static constexpr int SmemOffset(bool upper, int k)
+    {
+        int t = upper ? SmemSlots() / 2 : 0;
+        for (int j = 0; j < k; ++j) if (InSmem(j)) t += Width(j);
+        return t;
+    }
+    // index of a global stage among the global stages (lower first)
+    static constexpr int GIdx(bool upper, int k)
+    {
+        int t = upper ? NumGlobalStages() / 2 : 0;
+        for (int j = 0; j < k; ++j) if (!InSmem(j)) ++t;
         return t;
     }
     static constexpr int NumGlobalStages()
@@ -68,23 +92,11 @@ template <int FT> struct FLayout
         for (int k = 0; k < nStages; ++k) if (!InSmem(k)) ++t;
         return 2 * t;
     }
-    // index of a global stage among the global stages (lower first)
-    static constexpr int GIdx(bool upper, int k)
+    static constexpr int WindowSlots()
     {
         int t = 0;
-        for (int u = 0; u < 2; ++u)
-            for (int j = 0; j < nStages; ++j)
-            {
-                if (u == (upper ? 1 : 0) && j == k) return t;
-                if (!InSmem(j)) ++t;
-            }
+        for (int k = 0; k < nStages; ++k) t += 4 * Width(k);
         return t;
-    }
-    static constexpr int GlobalRingSlots()
-    {
-        int t = 0;
-        for (int k = 0; k < nStages; ++k) if (!InSmem(k)) t += 2 * Width(k);
-        return 2 * t;
     }
     static constexpr int CumStride(int i)
     {
@@ -93,12 +105,10 @@ template <int FT> struct FLayout
         return c;
     }
     static constexpr int AggStride() { return CumStride(S::n - 1); }
-    // int16 state: smem-resident arrays, global-resident arrays, then (P, c)
-    // per stage, then latData, latRaw, masks.
-    static constexpr int SlotSmem() { return 0; }
-    static constexpr int SlotGlobal() { return SmemSlots(); }
-    static constexpr int SlotPC(bool upper, int k) { return SmemSlots() + GlobalRingSlots() + 2 * Idx(upper, k); }
-    static constexpr int SlotLatData() { return SmemSlots() + GlobalRingSlots() + 4 * nStages; }
+    // int16 state: the windows, then (P, c) per stage, then latData, latRaw,
+    // masks.
+    static constexpr int SlotPC(bool upper, int k) { return WindowSlots() + 2 * Idx(upper, k); }
+    static constexpr int SlotLatData() { return WindowSlots() + 4 * nStages; }
     static constexpr int NumI16Slots() { return SlotLatData() + 3; }
 };
 
@@ -135,119 +145,41 @@ template <bool IsMax> __device__ __forceinline__ uint32_t Op2(uint32_t a, uint32
 }
 template <bool IsMax> constexpr uint32_t Identity2() { return IsMax ? 0x80008000u : 0x7fff7fffu; }
 
-// One van Herk/Gil-Werman window stage for a ZMW pair.  The output for each
-// input is the extremum of the W previous inputs (TraceFilters.cpp:11-57 with
-// the window state of WindowBuffer.h; the initial window holds W zeros).  The
-// state is the suffix extrema S of the previous block of W inputs, the
-// running extremum P of the current block and the current block's inputs B;
-// the output at block position c is op(S[c], P).  `base` points at S[0] of
-// this thread and `stride` separates consecutive array elements.
-template <int W, bool IsMax>
-__device__ __forceinline__ uint32_t StageStep2(uint32_t* base, int stride, uint32_t& P, int& counter, uint32_t x)
-{
-    uint32_t* S = base;
-    uint32_t* B = base + W * stride;
-    const int c = counter;
-    const uint32_t y = Op2<IsMax>(S[c * stride], P);
-    B[c * stride] = x;
-    P = Op2<IsMax>(P, x);
-    if (c + 1 == W)
-    {
-        // New suffix extrema of the completed block.
-        uint32_t acc = x;
-        S[(W - 1) * stride] = acc;
-#pragma unroll 1
-        for (int j = W - 2; j >= 0; --j)
-        {
-            acc = Op2<IsMax>(B[j * stride], acc);
-            S[j * stride] = acc;
-        }
-        P = Identity2<IsMax>();
-        counter = 0;
-    }
-    else
-    {
-        counter = c + 1;
-    }
-    return y;
-}
-
-// Global-memory window stage with S[counter] held in a register, loaded one
-// call ahead of its use (S changes only when a block completes), so the
-// stage never waits for memory on its critical path.  At a block's end the
-// inputs are read in batches of 4 before the batch's results are stored.
-template <int W, bool IsMax>
-__device__ __forceinline__ uint32_t StageStepG2(uint32_t* base, int stride, uint32_t& P, int& counter,
-                                                uint32_t& sNext, uint32_t x)
-{
-    uint32_t* S = base;
-    uint32_t* B = base + W * stride;
-    const int c = counter;
-    const uint32_t y = Op2<IsMax>(sNext, P);
-    B[c * stride] = x;
-    P = Op2<IsMax>(P, x);
-    if (c + 1 == W)
-    {
-        uint32_t acc = x;
-        S[(W - 1) * stride] = acc;
-        constexpr int kBatch = 4;
-#pragma unroll 1
-        for (int j0 = W - 2; j0 >= 0; j0 -= kBatch)
-        {
-            uint32_t b[kBatch];
-#pragma unroll
-            for (int q = 0; q < kBatch; ++q)
-                if (j0 - q >= 0) b[q] = B[(j0 - q) * stride];
-#pragma unroll
-            for (int q = 0; q < kBatch; ++q)
-                if (j0 - q >= 0)
-                {
-                    acc = Op2<IsMax>(b[q], acc);
-                    S[(j0 - q) * stride] = acc;
-                }
-        }
-        sNext = acc;      // S[0]
-        P = Identity2<IsMax>();
-        counter = 0;
-    }
-    else
-    {
-        counter = c + 1;
-        sNext = S[(c + 1) * stride];
-    }
-    return y;
-}
-
+// One scale of both filters for a ZMW pair: the lower filter's two window
+// stages and the upper filter's two, each van Herk/Gil-Werman.  A stage's
+// output for each input is the extremum of the W previous inputs
+// (TraceFilters.cpp:11-57 with the window state of WindowBuffer.h; the initial
+// window holds W zeros).  Its state is the suffix extrema S of the previous
+// block of W inputs, the running extremum P of the current block and the
+// current block's inputs B; the output at block position c is op(S[c], P).
+// The four stages are fed at the same frames and so share c: one counter, one
+// address and one end-of-block pass for the four (four independent chains)
+// instead of four of each.
+//
+// A scale that runs every frame or every other frame keeps its windows in
+// shared memory, S and B in one array (see FLayout).  The last scale's live in
+// global memory with S[c] loaded into a register one call (16 frames) ahead of
+// its use (S changes only when a block completes), so the stage never waits
+// for memory on its critical path.  Measured on 4096 lanes x 512 frames,
+// MultiScaleLarge: 17-wide windows in global memory 654 us, in shared memory 455
+// us; with S and B apart they would leave room for 7 blocks a SM instead of 14.
 struct StageMem2
 {
-    uint32_t* smem;     // this thread's column in shared memory
-    int sstride;        // blockDim.x
-    uint32_t* gmem;     // this pair's column of the global-resident arrays
-    int gstride;        // nZmw / 2
-    uint32_t* sNext;    // per global stage: S[counter], loaded ahead
+    uint32_t* smem;     // this thread's column in shared memory (stride kBlPairs)
+    uint32_t* gmem;     // this pair's column of the saved state, used in place
+    size_t gstride;     // nZmw / 2
+    uint32_t* sNext;    // per global stage: S[c], loaded ahead
 };
 
-// Filter state of one thread: P of every stage (a ZMW pair) and the lane's
-// block counters.
+constexpr int kBlPairs = kLane / 2;       // threads per lane
+
+// Filter state of one thread: P of every stage (a ZMW pair) and the block
+// counter of every scale.
 template <int FT> struct PairState
 {
     uint32_t P[2 * FLayout<FT>::nStages];
-    int c[2 * FLayout<FT>::nStages];
+    int c[FSpec<FT>::n];
 };
-
-template <int FT, bool Upper, int K>
-__device__ __forceinline__ uint32_t Stage2(const StageMem2& m, PairState<FT>& ps, uint32_t x)
-{
-    using Lay = FLayout<FT>;
-    constexpr int W = Lay::Width(K);
-    constexpr int off = Lay::Offset(Upper, K);
-    constexpr int i = Lay::Idx(Upper, K);
-    if constexpr (Lay::InSmem(K))
-        return StageStep2<W, Lay::IsMax(Upper, K)>(m.smem + off * m.sstride, m.sstride, ps.P[i], ps.c[i], x);
-    else
-        return StageStepG2<W, Lay::IsMax(Upper, K)>(m.gmem + (size_t)off * m.gstride, m.gstride, ps.P[i], ps.c[i],
-                                                    m.sNext[Lay::GIdx(Upper, K)], x);
-}
 
 // sNext of every global-memory stage of one filter from the saved state
 // (compile-time recursion: the stage layout tables are host constants).
@@ -258,24 +190,130 @@ __device__ __forceinline__ void LoadSNext2(const StageMem2& m, const PairState<F
     if constexpr (K < Lay::nStages)
     {
         if constexpr (!Lay::InSmem(K))
-        {
-            constexpr int i = Lay::Idx(Upper, K);
-            constexpr int off = Lay::Offset(Upper, K);
-            m.sNext[Lay::GIdx(Upper, K)] = m.gmem[((size_t)off + (size_t)ps.c[i]) * (size_t)m.gstride];
-        }
+            m.sNext[Lay::GIdx(Upper, K)] = m.gmem[(size_t)(Lay::SlotWindow(Upper, K) + ps.c[K / 2]) * m.gstride];
         LoadSNext2<FT, Upper, K + 1>(m, ps);
     }
 }
 
-template <int FT, bool Upper, int Scale>
-__device__ __forceinline__ uint32_t RunScale2(const StageMem2& m, PairState<FT>& ps, uint32_t x)
+// Shared-memory windows from (Save: to) the saved state, where S and B have
+// slots of their own: the part of each that the block position needs.
+template <int FT, bool Upper, int K, bool Save>
+__device__ __forceinline__ void CopyWindows(uint32_t* smem, uint32_t* state, size_t nPair, const PairState<FT>& ps)
 {
-    const uint32_t y = Stage2<FT, Upper, 2 * Scale>(m, ps, x);
-    return Stage2<FT, Upper, 2 * Scale + 1>(m, ps, y);
+    using Lay = FLayout<FT>;
+    if constexpr (K < Lay::nStages)
+    {
+        if constexpr (Lay::InSmem(K))
+        {
+            constexpr int W = Lay::Width(K);
+            const int c = ps.c[K / 2];
+#pragma unroll 17
+            for (int j = 0; j < W; ++j)
+            {
+                uint32_t& at = state[(size_t)(Lay::SlotWindow(Upper, K) + j + (j < c ? W : 0)) * nPair];
+                uint32_t& w = smem[(Lay::SmemOffset(Upper, K) + j) * kBlPairs];
+                if (Save) at = w;
+                else w = at;
+            }
+        }
+        CopyWindows<FT, Upper, K + 1, Save>(smem, state, nPair, ps);
+    }
+    else if constexpr (!Upper) CopyWindows<FT, true, 0, Save>(smem, state, nPair, ps);
 }
 
-// Feeds one frame through one multi-scale filter; returns true and the
-// envelope value when the last stage produced an output.  Cumulative strides
+// lo and up enter as the scale's inputs and leave as its outputs.
+template <int FT, int Scale>
+__device__ __forceinline__ void RunScale2(const StageMem2& m, PairState<FT>& ps, uint32_t& lo, uint32_t& up)
+{
+    using Lay = FLayout<FT>;
+    constexpr int K0 = 2 * Scale, K1 = K0 + 1, W = Lay::Width(K0);
+    constexpr bool smem = Lay::InSmem(K0);
+    // stages: lower first, lower second, upper first, upper second
+    constexpr int off[4] = {smem ? Lay::SmemOffset(false, K0) : Lay::SlotWindow(false, K0),
+                            smem ? Lay::SmemOffset(false, K1) : Lay::SlotWindow(false, K1),
+                            smem ? Lay::SmemOffset(true, K0) : Lay::SlotWindow(true, K0),
+                            smem ? Lay::SmemOffset(true, K1) : Lay::SlotWindow(true, K1)};
+    constexpr int pi[4] = {Lay::Idx(false, K0), Lay::Idx(false, K1), Lay::Idx(true, K0), Lay::Idx(true, K1)};
+    constexpr int gi[4] = {Lay::GIdx(false, K0), Lay::GIdx(false, K1), Lay::GIdx(true, K0), Lay::GIdx(true, K1)};
+    constexpr bool isMax[4] = {Lay::IsMax(false, K0), Lay::IsMax(false, K1), Lay::IsMax(true, K0),
+                               Lay::IsMax(true, K1)};
+    auto op = [](bool mx, uint32_t a, uint32_t b) { return mx ? MaxS16x2(a, b) : MinS16x2(a, b); };
+    const size_t stride = smem ? (size_t)kBlPairs : m.gstride;
+    uint32_t* base = smem ? m.smem : m.gmem;
+    auto S = [&](int i, int j) -> uint32_t& { return base[(size_t)(off[i] + j) * stride]; };
+    auto B = [&](int i, int j) -> uint32_t& { return base[(size_t)(off[i] + (smem ? 0 : W) + j) * stride]; };
+    const int c = ps.c[Scale];
+    uint32_t x[4];
+    x[0] = lo;
+    x[2] = up;
+#pragma unroll
+    for (int u = 0; u < 4; u += 2)
+    {
+        uint32_t in = x[u];
+#pragma unroll
+        for (int i = u; i < u + 2; ++i)
+        {
+            x[i] = in;
+            uint32_t s;
+            if constexpr (smem) s = S(i, c);
+            else s = m.sNext[gi[i]];
+            in = op(isMax[i], s, ps.P[pi[i]]);
+            B(i, c) = x[i];
+            ps.P[pi[i]] = op(isMax[i], ps.P[pi[i]], x[i]);
+        }
+        (u ? up : lo) = in;
+    }
+    if (c + 1 == W)
+    {
+        // New suffix extrema of the completed blocks.
+        uint32_t acc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            acc[i] = x[i];
+            S(i, W - 1) = acc[i];
+        }
+        constexpr int kBatch = 2;       // inputs read before the batch's results are stored
+#pragma unroll 1
+        for (int j0 = W - 2; j0 >= 0; j0 -= kBatch)
+        {
+            uint32_t b[kBatch][4];
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (W % kBatch == 1 || j0 - q >= 0) b[q][i] = B(i, j0 - q);
+#pragma unroll
+            for (int q = 0; q < kBatch; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (W % kBatch == 1 || j0 - q >= 0)
+                    {
+                        acc[i] = op(isMax[i], b[q][i], acc[i]);
+                        S(i, j0 - q) = acc[i];
+                    }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+        {
+            if constexpr (!smem) m.sNext[gi[i]] = acc[i];      // S[0]
+            ps.P[pi[i]] = isMax[i] ? Identity2<true>() : Identity2<false>();
+        }
+        ps.c[Scale] = 0;
+    }
+    else
+    {
+        ps.c[Scale] = c + 1;
+        if constexpr (!smem)
+        {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) m.sNext[gi[i]] = S(i, c + 1);
+        }
+    }
+}
+
+// Feeds one frame through both multi-scale filters; returns true and the
+// envelope values when the last scale produced an output.  Cumulative strides
 // are 1, 2 or 16 and chunks are multiples of 16 frames, so the scales that
 // run depend only on the frame's phase within its 16-frame block:
 // Phase 0 = first frame of the block, 1 = other even frames, 2 = odd frames.
@@ -285,27 +323,31 @@ __host__ __device__ constexpr bool ScaleRuns(int cumStride)
     return cumStride == 1 || (cumStride == 2 && Phase <= 1) || (cumStride == 16 && Phase == 0);
 }
 
-template <int FT, bool Upper, int Phase>
-__device__ __forceinline__ bool FeedFilter2(uint32_t x, const StageMem2& m, PairState<FT>& ps, uint32_t& out)
+template <int FT, int Phase>
+__device__ __forceinline__ bool FeedFilters2(uint32_t x, const StageMem2& m, PairState<FT>& ps, uint32_t& lo,
+                                             uint32_t& up)
 {
     using S = FSpec<FT>;
     using Lay = FLayout<FT>;
     static_assert(Lay::CumStride(0) <= 2 && (S::n < 2 || Lay::CumStride(1) <= 16) && Lay::AggStride() == 16,
                   "phase scheme needs cumulative strides 1|2, 2, 16");
+    lo = up = x;
     if constexpr (!ScaleRuns<Phase>(Lay::CumStride(0))) return false;
-    uint32_t y = RunScale2<FT, Upper, 0>(m, ps, x);
-    if constexpr (S::n > 1)
+    else
     {
+        RunScale2<FT, 0>(m, ps, lo, up);
         if constexpr (!ScaleRuns<Phase>(Lay::CumStride(1))) return false;
-        y = RunScale2<FT, Upper, 1>(m, ps, y);
+        else
+        {
+            RunScale2<FT, 1>(m, ps, lo, up);
+            if constexpr (S::n > 2)
+            {
+                if constexpr (!ScaleRuns<Phase>(Lay::CumStride(2))) return false;
+                else RunScale2<FT, 2>(m, ps, lo, up);
+            }
+            return true;
+        }
     }
-    if constexpr (S::n > 2)
-    {
-        if constexpr (!ScaleRuns<Phase>(Lay::CumStride(2))) return false;
-        y = RunScale2<FT, Upper, 2>(m, ps, y);
-    }
-    out = y;
-    return true;
 }
 
 // Initial filter state: every window holds W zeros (S = 0), the current block
@@ -326,8 +368,6 @@ __global__ void BaselinerInitKernel(int16_t* st16, float* st32, int lanes)
     st32[(size_t)2 * nZmw + g] = 2.0f;     // blSigmaEma_ initial value
 }
 
-constexpr int kBlPairs = kLane / 2;       // threads per lane
-
 // Reads the trace value pair of frame t.
 template <typename TIn>
 __device__ __forceinline__ uint32_t LoadPair(const TIn* tr, int t)
@@ -343,16 +383,47 @@ __device__ __forceinline__ uint32_t LoadPair(const TIn* tr, int t)
     }
 }
 
-__device__ __forceinline__ float2 PairToFloat(uint32_t p) { return f2((float)Lo16(p), (float)Hi16(p)); }
-
-// x - pedestal with int16 wrap-around, per half.
-__device__ __forceinline__ uint32_t SubPed(uint32_t x, int16_t ped)
+// Both int16 values as floats, exact: with the sign bit flipped a value is
+// v + 32768 in 16 bits, which as the low half of 2^23's bits is the float
+// 2^23 + 32768 + v.  (Three ALU instructions and a packed addition instead of
+// two conversions at a quarter of the rate.)
+__device__ __forceinline__ float2 PairToFloat(uint32_t p)
 {
-    return Pack16(i16_wrap(Lo16(x) - ped), i16_wrap(Hi16(x) - ped));
+    const uint32_t u = p ^ 0x80008000u;
+    return add2(f2(__uint_as_float(__byte_perm(u, 0x4b000000u, 0x7610)),
+                   __uint_as_float(__byte_perm(u, 0x4b000000u, 0x7632))),
+                f2(-(8388608.0f + 32768.0f)));
+}
+
+// x - pedestal with int16 wrap-around, per half (negPed: both halves -pedestal).
+__device__ __forceinline__ uint32_t SubPed(uint32_t x, uint32_t negPed)
+{
+    uint32_t r;
+    asm("add.s16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(negPed));
+    return r;
+}
+
+// Reference float -> int16 conversion of both values (to_i16_wrap) when both
+// are below 2^22 in magnitude: added to 1.5 * 2^23 they round to the nearest
+// even integer, whose low 16 bits are the sum's.
+__device__ __forceinline__ uint32_t RoundPair(float2 v)
+{
+    const float2 m = add2(v, f2(12582912.0f));
+    return __byte_perm(__float_as_uint(m.x), __float_as_uint(m.y), 0x5410);
+}
+// The same for any values.
+__device__ __noinline__ uint32_t RoundPairGeneral(float2 v) { return Pack16(to_i16_wrap(v.x), to_i16_wrap(v.y)); }
+
+// a < b ? 1 : 0 (0 when either is NaN).
+__device__ __forceinline__ float LessAsFloat(float a, float b)
+{
+    float r;
+    asm("set.lt.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
 template <int FT, typename TIn, bool Mapped>
-__global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a, KParams k)
+__global__ void __launch_bounds__(kBlPairs, 16) BaselinerKernel(BaselinerArgs a, KParams k)
 {
     using Lay = FLayout<FT>;
     LaneMap map = a.map;
@@ -372,14 +443,11 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
     // Window state: narrow windows in shared memory (one column per thread),
     // wide ones used in place in global memory.
     extern __shared__ uint32_t blSmem2[];
-    constexpr int SS = Lay::SmemSlots();
     constexpr int NG = Lay::NumGlobalStages() > 0 ? Lay::NumGlobalStages() : 1;
     uint32_t sNext[NG];
     const uint32_t* st = reinterpret_cast<const uint32_t*>(a.st16);
     uint32_t* stw = reinterpret_cast<uint32_t*>(a.st16);
-    const StageMem2 mem{blSmem2 + t, kBlPairs, stw + (size_t)Lay::SlotGlobal() * nPair + gp, nPair, sNext};
-#pragma unroll 32
-    for (int i = 0; i < SS; ++i) blSmem2[i * kBlPairs + t] = st[(size_t)(Lay::SlotSmem() + i) * nPair + gp];
+    const StageMem2 mem{blSmem2 + t, stw + gp, (size_t)nPair, sNext};
     PairState<FT> fs;
 #pragma unroll
     for (int i = 0; i < 2 * Lay::nStages; ++i)
@@ -387,16 +455,19 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
         const bool up = i >= Lay::nStages;
         const int kk = up ? i - Lay::nStages : i;
         fs.P[i] = st[(size_t)Lay::SlotPC(up, kk) * nPair + gp];
-        fs.c[i] = Lo16(st[(size_t)(Lay::SlotPC(up, kk) + 1) * nPair + gp]);   // the same for every ZMW
+        // the same for every ZMW and every stage of a scale
+        if (!up && kk % 2 == 0) fs.c[kk / 2] = Lo16(st[(size_t)(Lay::SlotPC(up, kk) + 1) * nPair + gp]);
     }
+    CopyWindows<FT, false, 0, false>(blSmem2 + t, stw + gp, (size_t)nPair, fs);
     // S[counter] of every global stage
     LoadSNext2<FT, false, 0>(mem, fs);
     LoadSNext2<FT, true, 0>(mem, fs);
     uint32_t latData = st[(size_t)Lay::SlotLatData() * nPair + gp];
     uint32_t latRaw = st[(size_t)(Lay::SlotLatData() + 1) * nPair + gp];
     const uint32_t mbits = st[(size_t)(Lay::SlotLatData() + 2) * nPair + gp];
-    bool latL0 = mbits & 1, latH10 = (mbits >> 1) & 1, latH20 = (mbits >> 2) & 1;
-    bool latL1 = (mbits >> 16) & 1, latH11 = (mbits >> 17) & 1, latH21 = (mbits >> 18) & 1;
+    // 1 where the previous frame was in the baseline (its threshold and its
+    // latent copy), else 0; hp2: the frame before it
+    float2 hp1 = f2((mbits & 3u) == 3u ? 1.0f : 0.0f, ((mbits >> 16) & 3u) == 3u ? 1.0f : 0.0f), hp2 = hp1;
     const float2* st32 = reinterpret_cast<const float2*>(a.st32);
     float2 uemaSum = st32[(size_t)0 * nPair + gp];
     float2 uemaWeight = st32[(size_t)1 * nPair + gp];
@@ -404,15 +475,15 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
     const float2 nz = f2(k.negZero);
 
     // Per-chunk BaselinerStatAccumulator (fresh each chunk, offset 0).  The
-    // frame counts are the same for both ZMWs.
-    float c_m0 = 0.0f;
+    // sample counts are F and F / 16; the front buffer (the first four
+    // samples) is the latent frame and the chunk's first three outputs, read
+    // back at the end.
     float2 c_m1 = f2(0.0f), c_m2 = f2(0.0f), c_acm2 = f2(0.0f);
-    float2 fb0 = f2(0.0f), fb1 = f2(0.0f), fb2 = f2(0.0f), fb3 = f2(0.0f);
-    float2 q0 = f2(0.0f), q1 = f2(0.0f), q2 = f2(0.0f), q3 = f2(0.0f);     // back buffer as a FIFO, q0 oldest
-    int nAdded = 0;
+    const uint32_t firstData = latData;
+    float2 back[4] = {f2(0.0f), f2(0.0f), f2(0.0f), f2(0.0f)};     // last four samples, back[f % 4] of frame f
+    float2 latV = PairToFloat(latData), latRawV = PairToFloat(latRaw);
     uint32_t tmin = 0x7fff7fffu, tmax = 0x80008000u;
     float2 b_m0 = f2(0.0f), b_m1 = f2(0.0f), b_m2 = f2(0.0f), rawSum = f2(0.0f);
-    float g_m0 = 0.0f;
     float2 g_m1 = f2(0.0f), g_m2 = f2(0.0f);
 
     const TIn* tr;
@@ -420,30 +491,38 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
     if constexpr (std::is_same_v<TIn, uint8_t>) tr = (ps ? ps->trace8 : a.trace8) + inOff + z;
     else tr = (ps ? ps->trace : a.trace) + inOff + z;
     uint32_t* out = reinterpret_cast<uint32_t*>(a.out + map.Block(lane, F) + z);
-    const int16_t ped = (int16_t)k.pedestal;
+    const uint32_t negPed = Pack16(i16_wrap(-k.pedestal), i16_wrap(-k.pedestal));
     const float2 scaler = f2(k.scaler);
-    float2 sub = f2(0.0f);
+    const bool scalerOk = fabsf(k.scaler) <= 63.0f;     // |x scaler| < 2^21
+    float2 negSub = f2(0.0f), thr = f2(0.0f);
+    bool inRange = false;
 
     // Frames go in blocks of 16 (the aggregate stride): the first frame of a
     // block, the other even frames and the odd frames each get their own
-    // specialisation of the frame body, with the trace loaded two frames ahead.
-    // Even frames take their value from xEven and odd frames from xOdd, each
+    // specialisation of the frame body (four frames a loop turn, the period
+    // of the back buffer), with the trace loaded two frames ahead.  Even
+    // frames take their value from xEven and odd frames from xOdd, each
     // refilled right after use: no register is copied while its load is in
-    // flight.
+    // flight.  Two loads in flight a warp do not cover the latency of DRAM at
+    // 14 warps a SM, so each block prefetches the block after the next: the
+    // lane's frames are consecutive lines, one a thread (708 -> 672 us on the
+    // case above, 243 -> 192 us on TwoScaleMedium, 2048 lanes).
     static_assert(Lay::AggStride() == 16, "block size must be the aggregate stride");
+    const TIn* lines = tr - z;
+    if (t < F) PrefetchL1(lines + (size_t)t * kLane);
     uint32_t xEven = LoadPair(tr, 0), xOdd = LoadPair(tr, 1);
-    auto frame = [&](auto phaseTag, int f) {
+    auto frame = [&](auto phaseTag, auto slotTag, int f) {
         constexpr int Ph = decltype(phaseTag)::value;
+        constexpr int Slot = decltype(slotTag)::value;
         uint32_t& slot = (Ph == 2) ? xOdd : xEven;      // phase 2 = odd frames
         const uint32_t x = slot;
         if (f + 2 < F) slot = LoadPair(tr, f + 2);
-        uint32_t lo = 0, up = 0;
-        const bool haveL = FeedFilter2<FT, false, Ph>(x, mem, fs, lo);
-        FeedFilter2<FT, true, Ph>(x, mem, fs, up);
+        uint32_t lo, up;
+        const bool haveL = FeedFilters2<FT, Ph>(x, mem, fs, lo, up);
         if (haveL)
         {
             // GetSmoothedBlEstimate (HostMultiScaleBaseliner.cpp:179-212)
-            const uint32_t lv = SubPed(lo, ped), uv = SubPed(up, ped);
+            const uint32_t lv = SubPed(lo, negPed), uv = SubPed(up, negPed);
             constexpr float minSigma = .288675135f;
             const float ma = k.meanEmaAlpha, sa = k.sigmaEmaAlpha;
             float2 sigma;
@@ -461,82 +540,87 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
             uemaSum = f2(mx ? newSum.x : uemaSum.x, my ? newSum.y : uemaSum.y);
             sigmaEma = f2(mx ? newSigmaEma.x : sigmaEma.x, my ? newSigmaEma.y : sigmaEma.y);
             const float2 est = f2(uemaSum.x / uemaWeight.x, uemaSum.y / uemaWeight.y);
-            sub = mulz2(est, scaler, nz);      // feeds the subtraction of every frame
+            const float2 sub = mulz2(est, scaler, nz);      // feeds the subtraction of every frame
+            negSub = f2(-sub.x, -sub.y);
+            thr = mul2(mul2(f2(4.5f), sigmaEma), scaler);
+            inRange = scalerOk & (fabsf(sub.x) < 2097152.0f) & (fabsf(sub.y) < 2097152.0f);
             // AddSampleBackground (BaselinerStatAccumulator.cpp:56-60)
             const float2 bg = f2((float)to_i16_wrap(sub.x), (float)to_i16_wrap(sub.y));
-            g_m0 += 1.0f;
             g_m1 = add2(g_m1, bg);
             g_m2 = add2(g_m2, mulz2(bg, bg, nz));
         }
-        const uint32_t xp = SubPed(x, ped);
-        const float2 rs = mulz2(PairToFloat(xp), scaler, nz);
-        const float2 d = add2(rs, f2(-sub.x, -sub.y));
-        const int16_t blsX = to_i16_wrap(d.x), blsY = to_i16_wrap(d.y);
-        const uint32_t bls = Pack16(blsX, blsY);
+        const float2 rs = mulz2(PairToFloat(SubPed(x, negPed)), scaler, nz);
+        const float2 d = add2(rs, negSub);
+        uint32_t bls = RoundPair(d), raw = RoundPair(rs);
+        if (!inRange)
+        {
+            bls = RoundPairGeneral(d);
+            raw = RoundPairGeneral(rs);
+        }
         out[(size_t)f * (kLane / 2)] = bls;
-        const uint32_t raw = Pack16(to_i16_wrap(rs.x), to_i16_wrap(rs.y));
 
-        // AddToBaselineStats (HostMultiScaleBaseliner.cpp:148-176)
-        const float2 thr = mul2(mul2(f2(4.5f), sigmaEma), scaler);
-        const float2 fb = f2((float)blsX, (float)blsY);
-        const bool hpX = fb.x < thr.x, hpY = fb.y < thr.y;
-        const bool mX = latH10 & latL0 & hpX, mY = latH11 & latL1 & hpY;
-        latL0 = hpX; latL1 = hpY;
-        latH20 = latH10; latH21 = latH11;
-        latH10 = hpX; latH11 = hpY;
+        // AddToBaselineStats (HostMultiScaleBaseliner.cpp:148-176): the latent
+        // frame is a baseline sample when it and the current one are below
+        // the threshold.  As a factor of 1 or 0 in one fma per sum: v m + sum
+        // rounds as v + sum for 1 and leaves the sum for 0.
+        const float2 fb = PairToFloat(bls);
+        const float2 hp = f2(LessAsFloat(fb.x, thr.x), LessAsFloat(fb.y, thr.y));
+        const float2 m = mul2(hp1, hp);
+        hp2 = hp1;
+        hp1 = hp;
         {
             // BaselinerStatAccumulator::AddSample(latRaw, latData, m)
-            const float2 v = PairToFloat(latData);
-            if (nAdded < 4)
-            {
-                if (nAdded == 0) fb0 = v; else if (nAdded == 1) fb1 = v; else if (nAdded == 2) fb2 = v; else fb3 = v;
-            }
-            c_acm2 = add2(c_acm2, mulz2(q0, v, nz));
-            q0 = q1; q1 = q2; q2 = q3; q3 = v;
-            ++nAdded;
-            c_m0 += 1.0f;
+            const float2 v = latV;
+            c_acm2 = add2(c_acm2, mulz2(back[Slot], v, nz));
+            back[Slot] = v;
             c_m1 = add2(c_m1, v);
             const float2 vv = mulz2(v, v, nz);
             c_m2 = add2(c_m2, vv);
             tmin = MinS16x2(latData, tmin);
             tmax = MaxS16x2(latData, tmax);
-            const float2 a0 = add2(b_m0, f2(1.0f)), a1 = add2(b_m1, v), a2 = add2(b_m2, vv);
-            b_m0 = f2(mX ? a0.x : b_m0.x, mY ? a0.y : b_m0.y);
-            b_m1 = f2(mX ? a1.x : b_m1.x, mY ? a1.y : b_m1.y);
-            b_m2 = f2(mX ? a2.x : b_m2.x, mY ? a2.y : b_m2.y);
-            rawSum = add2(rawSum, f2((float)(mX ? Lo16(latRaw) : (int16_t)0), (float)(mY ? Hi16(latRaw) : (int16_t)0)));
+            b_m0 = add2(b_m0, m);
+            b_m1 = fma2(m, v, b_m1);
+            b_m2 = fma2(m, vv, b_m2);
+            rawSum = fma2(m, latRawV, rawSum);
         }
         latRaw = raw;
+        latRawV = PairToFloat(raw);
         latData = bls;
+        latV = fb;
     };
+    using P0 = std::integral_constant<int, 0>;
+    using P1 = std::integral_constant<int, 1>;
+    using P2 = std::integral_constant<int, 2>;
+    using P3 = std::integral_constant<int, 3>;
 #pragma unroll 1
-    for (int t0 = 0; t0 < F; t0 += 16)
+    for (int f = 0; f < F; f += 4)
     {
-        frame(std::integral_constant<int, 0>{}, t0);
-#pragma unroll 1
-        for (int j = 1; j < 16; j += 2)
+        if ((f & 15) == 0)
         {
-            frame(std::integral_constant<int, 2>{}, t0 + j);
-            if (j + 1 < 16) frame(std::integral_constant<int, 1>{}, t0 + j + 1);
+            if (t < 16 && f + 32 + t < F) PrefetchL1(lines + (size_t)(f + 32 + t) * kLane);
+            frame(P0{}, P0{}, f);
         }
+        else frame(P1{}, P0{}, f);
+        frame(P2{}, P1{}, f + 1);
+        frame(P1{}, P2{}, f + 2);
+        frame(P2{}, P3{}, f + 3);
     }
 
     // Store state.
-#pragma unroll 8
-    for (int i = 0; i < SS; ++i) stw[(size_t)(Lay::SlotSmem() + i) * nPair + gp] = blSmem2[i * kBlPairs + t];
+    CopyWindows<FT, false, 0, true>(blSmem2 + t, stw + gp, (size_t)nPair, fs);
 #pragma unroll
     for (int i = 0; i < 2 * Lay::nStages; ++i)
     {
         const bool up = i >= Lay::nStages;
         const int kk = up ? i - Lay::nStages : i;
         stw[(size_t)Lay::SlotPC(up, kk) * nPair + gp] = fs.P[i];
-        stw[(size_t)(Lay::SlotPC(up, kk) + 1) * nPair + gp] = Pack16((int16_t)fs.c[i], (int16_t)fs.c[i]);
+        stw[(size_t)(Lay::SlotPC(up, kk) + 1) * nPair + gp] = Pack16((int16_t)fs.c[kk / 2], (int16_t)fs.c[kk / 2]);
     }
     stw[(size_t)Lay::SlotLatData() * nPair + gp] = latData;
     stw[(size_t)(Lay::SlotLatData() + 1) * nPair + gp] = latRaw;
-    stw[(size_t)(Lay::SlotLatData() + 2) * nPair + gp] =
-        Pack16((int16_t)((latL0 ? 1 : 0) | (latH10 ? 2 : 0) | (latH20 ? 4 : 0)),
-               (int16_t)((latL1 ? 1 : 0) | (latH11 ? 2 : 0) | (latH21 ? 4 : 0)));
+    // bits 0, 1: the last frame (latent and first history copy), 2: the one before
+    auto bits = [](float last, float before) { return (int16_t)((last != 0.0f ? 3 : 0) | (before != 0.0f ? 4 : 0)); };
+    stw[(size_t)(Lay::SlotLatData() + 2) * nPair + gp] = Pack16(bits(hp1.x, hp2.x), bits(hp1.y, hp2.y));
     float2* st32w = reinterpret_cast<float2*>(a.st32);
     st32w[(size_t)0 * nPair + gp] = uemaSum;
     st32w[(size_t)1 * nPair + gp] = uemaWeight;
@@ -546,18 +630,18 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
     hw_baseliner_stats& S = a.stats[lane];
     auto put = [&](float* arr, float2 v) { *reinterpret_cast<float2*>(arr + z) = v; };
     put(S.full_autocorr.basic_stats.offset, f2(0.0f));
-    put(S.full_autocorr.basic_stats.moment0, f2(c_m0));
+    put(S.full_autocorr.basic_stats.moment0, f2((float)F));
     put(S.full_autocorr.basic_stats.moment1, c_m1);
     put(S.full_autocorr.basic_stats.moment2, c_m2);
     put(S.full_autocorr.moment2, c_acm2);
-    const int fbi = nAdded < 4 ? nAdded : 4;
-    const int bbi = nAdded % 4;
-    put(S.full_autocorr.fbuf[0], fb0); put(S.full_autocorr.fbuf[1], fb1);
-    put(S.full_autocorr.fbuf[2], fb2); put(S.full_autocorr.fbuf[3], fb3);
-    // bBuf[(bbi + j) % 4] holds the j-th oldest of the last four samples.
-    const float2 qq[4] = {q0, q1, q2, q3};
+    // F is a multiple of 16: four samples in the front buffer, and the back
+    // buffer's next slot is 0, so slot j holds the j-th oldest of the last four
+    const int fbi = 4, bbi = 0;
+    put(S.full_autocorr.fbuf[0], PairToFloat(firstData));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) put(S.full_autocorr.bbuf[(bbi + j) % 4], qq[j]);
+    for (int j = 0; j < 3; ++j) put(S.full_autocorr.fbuf[j + 1], PairToFloat(out[(size_t)j * (kLane / 2)]));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) put(S.full_autocorr.bbuf[j], back[j]);
     *reinterpret_cast<uint16_t*>(&S.full_autocorr.bidx[0][z]) = (uint16_t)(fbi | (fbi << 8));
     *reinterpret_cast<uint16_t*>(&S.full_autocorr.bidx[1][z]) = (uint16_t)(bbi | (bbi << 8));
     *reinterpret_cast<uint32_t*>(&S.trace_min[z]) = tmin;
@@ -568,7 +652,7 @@ __global__ void __launch_bounds__(kBlPairs, 14) BaselinerKernel(BaselinerArgs a,
     put(S.baseline_stats.moment2, b_m2);
     put(S.raw_baseline_sum, rawSum);
     put(S.background_stats.offset, f2(0.0f));
-    put(S.background_stats.moment0, f2(g_m0));
+    put(S.background_stats.moment0, f2((float)(F / 16)));
     put(S.background_stats.moment1, g_m1);
     put(S.background_stats.moment2, g_m2);
 }

@@ -150,6 +150,122 @@ __device__ __forceinline__ float2 hw_expf2_np(float2 x, float2 nz)
     return out;
 }
 
+// d / b with r = RN(1/b): two corrections by the exact remainder (Markstein)
+// give the IEEE quotient when nothing under- or overflows.
+__device__ __forceinline__ float DivRcp(float d, float b, float r)
+{
+    float q = mul_rn(d, r);
+    q = fma_rn(fma_rn(-q, b, d), r, q);
+    return fma_rn(fma_rn(-q, b, d), r, q);
+}
+
+// int16 -> float, exactly: 1.5 x 2^23 + x has the bit pattern 0x4B400000 + x.
+__device__ __forceinline__ float I16ToFloat(int16_t x) { return __int_as_float(0x4B400000 + (int)x) - 12582912.0f; }
+
+// L1 prefetch of one address, no register result: brings in lines that the
+// next loads need sooner than their own distance can hide.
+__device__ __forceinline__ void PrefetchL1(const void* p) { asm volatile("prefetch.global.L1 [%0];" :: "l"(p)); }
+
+// Three-input maximum / minimum (one instruction on sm_100) for operands that
+// are never NaN and where the sign of a zero result does not matter.
+__device__ __forceinline__ float max3(float a, float b, float c)
+{
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c)
+{
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+// Packed addition rounded toward -infinity.
+__device__ __forceinline__ float2 add2_rd(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 pa, pb, pr;\n\tmov.b64 pa, {%2, %3};\n\tmov.b64 pb, {%4, %5};\n\t"
+        "add.rm.f32x2 pr, pa, pb;\n\tmov.b64 {%0, %1}, pr;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+// hw_expf without its special-case selects, for x in [-inf, 70] that is not
+// NaN: the same bits with about half the instructions and no conversion.
+//   * Arguments below -105 are raised to -105, where the routine's own
+//     arithmetic gives 0: exp(x) < 2^-150 rounds to 0 from
+//     x = -103.972084 down, which is the general routine's cut-off.
+//   * floor(t) is the addition of kExpMagic rounded toward -infinity: the sum
+//     lies in [2^23, 2^24), where a float's unit is 1.  Its low bits hold
+//     n + 127 + 24, so shifted to the exponent field they are 2^(n + 24) (0
+//     for n = -151, where the result is 0).
+//   * 2^n is applied as 2^(n + 24) and 2^-24 (n is in [-151, 101]): the
+//     second product rounds once, as the general routine's two factors do.
+// Equal to hw_expf on every float in [-inf, 70].
+constexpr float kExpMagic = 12582912.0f + 151.0f;      // 1.5 * 2^23 + 127 + 24
+constexpr float kExpDown = 5.9604644775390625e-08f;    // 2^-24
+__device__ __forceinline__ float hw_expf_fast(float x)
+{
+    const float xc = fmaxf(x, -105.0f);
+    const float m = __fadd_rd(fma_rn(xc, 1.44269504088896341f, 0.5f), kExpMagic);
+    const float z = m - kExpMagic;
+    float r = fma_rn(z, -0.693359375f, xc);
+    r = fma_rn(z, 2.12194440e-4f, r);
+    float p = fma_rn(1.9875691500e-4f, r, 1.3981999507e-3f);
+    p = fma_rn(p, r, 8.3334519073e-3f);
+    p = fma_rn(p, r, 4.1665795894e-2f);
+    p = fma_rn(p, r, 1.6666665459e-1f);
+    p = fma_rn(p, r, 5.0000001201e-1f);
+    const float r2 = mul_rn(r, r);
+    const float y = add_rn(fma_rn(p, r2, r), 1.0f);
+    return mul_rn(mul_rn(y, __int_as_float(__float_as_int(m) << 23)), kExpDown);
+}
+// Both components packed; every product that feeds an addition is an fma.
+__device__ __forceinline__ float2 hw_expf2_fast(float2 x, float2 nz)
+{
+    const float2 xc = f2(fmaxf(x.x, -105.0f), fmaxf(x.y, -105.0f));
+    const float2 m = add2_rd(fma2(xc, f2(1.44269504088896341f), f2(0.5f)), f2(kExpMagic));
+    const float2 z = add2(m, f2(-kExpMagic));
+    float2 r = fma2(z, f2(-0.693359375f), xc);
+    r = fma2(z, f2(2.12194440e-4f), r);
+    float2 p = fma2(f2(1.9875691500e-4f), r, f2(1.3981999507e-3f));
+    p = fma2(p, r, f2(8.3334519073e-3f));
+    p = fma2(p, r, f2(4.1665795894e-2f));
+    p = fma2(p, r, f2(1.6666665459e-1f));
+    p = fma2(p, r, f2(5.0000001201e-1f));
+    const float2 r2 = mul2(r, r);
+    const float2 y = add2(fma2(p, r2, r), f2(1.0f));
+    const float2 s = f2(__int_as_float(__float_as_int(m.x) << 23), __int_as_float(__float_as_int(m.y) << 23));
+    return mulz2(mul2(y, s), f2(kExpDown), nz);
+}
+
+// hw_logf without its special-case selects, equal to it on every positive
+// normal x: the same
+// decomposition x = f 2^e with f in [sqrt(1/2), sqrt(2)), found by one
+// subtraction of the bits of sqrt(1/2), and the same arithmetic after it.
+__device__ __forceinline__ float hw_logf_normal(float x)
+{
+    const int u = __float_as_int(x) - 0x3f3504f3;     // bits of 0.70710678f
+    const int e = u >> 23;
+    const float m = add_rn(__int_as_float(__float_as_int(x) - (u & (int)0xff800000)), -1.0f);
+    // (float)e, exact: the integer joins the unit digits of 1.5 * 2^23
+    const float fe = __int_as_float(0x4b400000 + e) - 12582912.0f;
+    const float z = mul_rn(m, m);
+    float y = 7.0376836292e-2f;
+    y = fma_rn(y, m, -1.1514610310e-1f);
+    y = fma_rn(y, m, 1.1676998740e-1f);
+    y = fma_rn(y, m, -1.2420140846e-1f);
+    y = fma_rn(y, m, 1.4249322787e-1f);
+    y = fma_rn(y, m, -1.6668057665e-1f);
+    y = fma_rn(y, m, 2.0000714765e-1f);
+    y = fma_rn(y, m, -2.4999993993e-1f);
+    y = fma_rn(y, m, 3.3333331174e-1f);
+    y = mul_rn(mul_rn(y, m), z);
+    y = fma_rn(fe, -2.12194440e-4f, y);
+    y = fma_rn(z, -0.5f, y);
+    return fma_rn(fe, 0.693359375f, add_rn(m, y));
+}
+
 // Device error word shared by the kernels of one launch: the first failing
 // check stores its code; the host reads it after the launch.
 struct ErrWord
