@@ -339,6 +339,20 @@ __device__ __forceinline__ void DmePrelude(const KParams& k, const hw_lane_model
     r.sExpectW = mul_rn(det.conf, k.pulseAmpReg);
 }
 
+// Arguments and results of the general E-step, which is not inlined.
+struct EmStepIo
+{
+    EmHist h;
+    EmVars v;
+    float* bpS;
+    float* tau0S;
+    float* facS;
+    float halfLog2pi, negZero;
+    float ci[5], mom1[5], varinv[5];
+    float ll;      // log-likelihood without the regularisation term
+    bool safe;
+};
+
 // One E-step over the 301 bin boundaries and 300 bins (DmeEmHost.cpp:363-492):
 // returns the log-likelihood, fills the mode totals ci, first moments mom1 and
 // inverse variances, and writes what the background-variance M-step needs to
@@ -356,17 +370,25 @@ __device__ __forceinline__ void DmePrelude(const KParams& k, const hw_lane_model
 //
 // kFull = false computes the log-likelihood alone (the same bits): no
 // responsibilities, sums or scratch, for the start that is only compared.
-template <bool kFull = true>
-__device__ __forceinline__ float EmEStep(const KParams& k, const EmHist& h, const EmVars& v, const EmReg& r,
-                                         float* bpS, float* tau0S, float* facS, float ci[5], float mom1[5],
-                                         float varinv[5], bool& safeOut)
+// This is the general form, for parameters of any value; EmEStep takes it
+// only when a ZMW of the warp has parameters outside the fast form's range.
+template <bool kFull>
+__device__ __noinline__ void EmEStepGeneric(EmStepIo& io)
 {
+    const EmHist& h = io.h;
+    const EmVars& v = io.v;
+    float* bpS = io.bpS;
+    float* tau0S = io.tau0S;
+    float* facS = io.facS;
+    float (&ci)[5] = io.ci;
+    float (&mom1)[5] = io.mom1;
+    float (&varinv)[5] = io.varinv;
     // Modes 0/1 and 2/3 run as packed pairs (hw_expf2, f32x2 arithmetic:
     // each component rounds exactly as the scalar operation), mode 4 alone.
     // Subtractions are additions of the exactly negated operand, and
     // pref - ((0.5 y) y) vinv is pref + ((-0.5 y) y) vinv: the same bits.
     const int z = h.z;
-    const float halfLog2pi = mul_rn(0.5f, k.logTwoPi);
+    const float halfLog2pi = io.halfLog2pi;
     float pref[5];
 #pragma unroll
     for (int i = 0; i < 5; ++i)
@@ -389,7 +411,7 @@ __device__ __forceinline__ float EmEStep(const KParams& k, const EmHist& h, cons
     const float2 vinv01 = f2(varinv[0], varinv[1]), vinv23 = f2(varinv[2], varinv[3]);
     const float2 nmu01 = f2(-v.mu[0], -v.mu[1]), nmu23 = f2(-v.mu[2], -v.mu[3]);
     const float pref4 = pref[4], vinv4 = varinv[4], mu4 = v.mu[4];
-    const float2 nz = f2(k.negZero);
+    const float2 nz = f2(io.negZero);
     float probSum = 0.0f, wps = 0.0f;
     float2 ci01 = f2(0.0f), ci23 = f2(0.0f), m01 = f2(0.0f), m23 = f2(0.0f);
     float ci4 = 0.0f, m4 = 0.0f;
@@ -492,11 +514,196 @@ __device__ __forceinline__ float EmEStep(const KParams& k, const EmHist& h, cons
     m23 = mulz2(m23, hb, nz);
     ci[0] = ci01.x; ci[1] = ci01.y; ci[2] = ci23.x; ci[3] = ci23.y; ci[4] = mul_rn(ci4, hb.x);
     mom1[0] = m01.x; mom1[1] = m01.y; mom1[2] = m23.x; mom1[3] = m23.y; mom1[4] = mul_rn(m4, hb.x);
-    float ll = wps - mul_rn(h.nSum, hw_logf(probSum));
+    io.ll = wps - mul_rn(h.nSum, hw_logf(probSum));
+    io.safe = safe;
+}
+
+// The E-step.  When every ZMW of the warp has finite parameters in an ordinary
+// range, each boundary is evaluated without the exponential's and logarithm's
+// special cases (their arguments cannot reach them: hw_expf_fast,
+// hw_logf_normal) and the loop ends with the last boundary that can change a
+// result; otherwise the general form runs.  Both give the same bits.
+//
+// Ordinary range (`fast`): the general form's `safe` with max(pref) < 40, so
+// densities stay below 5 e^40, boundaries and means below 1e6, so no moment
+// term overflows, and every exponent's square term below 1e30 at both ends of
+// the histogram, so all t are finite and llb - t and tmax - t are never NaN.
+//
+// End of the loop: after the warp's last occupied bin the bins only add to
+// probSum.  Beyond every mode's mean the densities fall (each step of t is
+// monotone in x), so a later bin adds at most max(binSize bp(b) (1 + 2^-10),
+// binProbMin); once that is at most 2^-27 probSum for every ZMW, adding it
+// leaves probSum unchanged (half a unit in its last place is above 2^-25
+// probSum) and the remaining boundaries have no effect.
+//
+// Bound by the FMA pipe (60%) and the dependent chain of a boundary; one thread
+// a ZMW, modes 0/1 and 2/3 as packed pairs.  A 4096-lane estimate took 18.5 ms
+// with the general form alone (84,900 thread instructions a ZMW and iteration)
+// and takes 11.5 ms (41,000); 37 lanes 3.24 -> 1.51 ms.  8 blocks a SM, where
+// nothing spills: 10 blocks with spills 12.3 ms, 7 blocks 11.5 ms.
+template <bool kFull = true>
+__device__ __forceinline__ float EmEStep(const KParams& k, const EmHist& h, const EmVars& v, const EmReg& r,
+                                         float* bpS, float* tau0S, float* facS, float ci[5], float mom1[5],
+                                         float varinv[5], bool& safeOut)
+{
+    const int z = h.z;
+    // the ZMWs taking this step together: a learned start's first iteration
+    // is for those of the warp that kept the reference start
+    const unsigned warp = __activemask();
+    const float halfLog2pi = mul_rn(0.5f, k.logTwoPi);
+    const float x0 = h.BinStart(0), xEnd = h.BinStart(kBins);
+    float pref[5];
+    bool fast = (fabsf(x0) < 1e6f) & (fabsf(xEnd) < 1e6f);
+    float muMax = v.mu[0];
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+    {
+        varinv[i] = 1.0f / v.var[i];
+        pref[i] = (hw_logf(v.rho[i]) - mul_rn(0.5f, hw_logf(v.var[i]))) - halfLog2pi;
+        const float y = fmaxf(fabsf(x0 - v.mu[i]), fabsf(xEnd - v.mu[i]));
+        fast &= isfinite(pref[i]) & (pref[i] < 40.0f) & (fabsf(v.mu[i]) < 1e6f) & isfinite(varinv[i]) &
+                (y * y * varinv[i] < 1e30f);
+        muMax = fmaxf(muMax, v.mu[i]);
+    }
+    float ll;
+    if (__all_sync(warp, fast))
+    {
+        safeOut = true;
+        const float2 pref01 = f2(pref[0], pref[1]), pref23 = f2(pref[2], pref[3]);
+        const float2 nhv01 = f2(-0.5f * varinv[0], -0.5f * varinv[1]), nhv23 = f2(-0.5f * varinv[2], -0.5f * varinv[3]);
+        const float2 nmu01 = f2(-v.mu[0], -v.mu[1]), nmu23 = f2(-v.mu[2], -v.mu[3]);
+        const float pref4 = pref[4], nhv4 = -0.5f * varinv[4], mu4 = v.mu[4];
+        const float2 nz = f2(k.negZero);
+        const float halfBin = mul_rn(0.5f, h.binSize);
+        float probSum = 0.0f, wps = 0.0f;
+        float2 ci01 = f2(0.0f), ci23 = f2(0.0f), m01 = f2(0.0f), m23 = f2(0.0f);
+        float ci4 = 0.0f, m4 = 0.0f;
+        float2 tp01 = f2(0.0f), tp23 = f2(0.0f);
+        float tp4 = 0.0f, bp = 0.0f, x = 0.0f, bf = 0.0f;
+
+        // cornerComp: the next boundary's x, mode exponents t and log density;
+        // (-0.5 y) y vinv = (y y) (-0.5 vinv): halving is exact
+        float2 t01, t23;
+        float t4, tmax;
+        auto corner = [&]() {
+            x = add_rn(h.lb, mul_rn(bf, h.binSize));
+            bf += 1.0f;
+            float2 y = add2(f2(x), nmu01);
+            t01 = add2(pref01, mulz2(mul2(y, y), nhv01, nz));
+            y = add2(f2(x), nmu23);
+            t23 = add2(pref23, mulz2(mul2(y, y), nhv23, nz));
+            const float y4 = x - mu4;
+            t4 = add_rn(pref4, mul_rn(mul_rn(y4, y4), nhv4));
+            tmax = max3(max3(t01.x, t01.y, t23.x), t23.y, t4);
+        };
+        auto logDensity = [&]() -> float {
+            const float2 ntmax = f2(-tmax);
+            const float2 e01 = hw_expf2_fast(add2(t01, ntmax), nz), e23 = hw_expf2_fast(add2(t23, ntmax), nz);
+            float se = add_rn(e01.x, e01.y);
+            se = add_rn(se, e23.x);
+            se = add_rn(se, e23.y);
+            se = add_rn(se, hw_expf_fast(t4 - tmax));
+            return add_rn(tmax, hw_logf_normal(se));
+        };
+        // a boundary between empty bins: its density only; far tails (llb <
+        // -104.3) have density 0
+        auto bare = [&]() {
+            corner();
+            bp = 0.0f;
+            if (tmax >= -106.0f) bp = hw_expf_fast(logDensity());
+        };
+        auto binProb = [&](float before) {
+            return fmaxf(mul_rn(halfBin, add_rn(before, bp)), h.binProbMin);
+        };
+        int b = 0;
+        for (; b < h.wLo; ++b)
+        {
+            const float before = bp;
+            bare();
+            if (b > 0) probSum = add_rn(probSum, binProb(before));
+        }
+        // the warp's occupied bins and their boundaries, without branches: a
+        // bin empty for this ZMW has factor 0 and adds 0 (every term is
+        // finite) to sums that never hold -0
+        uint32_t n = 0u, nNext = h.Count(b < kBins ? b : kBins - 1);
+        const int last = h.wHi + 1 > b ? h.wHi + 1 : b;
+#pragma unroll 1
+        for (; b <= last; ++b)
+        {
+            const float before = bp, xBefore = x;
+            corner();
+            const float llb = logDensity();
+            bp = hw_expf_fast(llb);
+            const float bpr = binProb(before);
+            probSum = b > 0 ? add_rn(probSum, bpr) : probSum;
+            const float nj = (float)n;      // of bin b - 1; 0 before the first occupied bin
+            n = nNext;
+            nNext = h.Count(b + 1 < kBins ? b + 1 : kBins - 1);
+            wps = add_rn(wps, mul_rn(nj, hw_logf_normal(bpr)));
+            if (kFull)
+            {
+                const float2 nllb = f2(-llb);
+                const float2 tau01 = hw_expf2_fast(add2(t01, nllb), nz), tau23 = hw_expf2_fast(add2(t23, nllb), nz);
+                const float tau4 = hw_expf_fast(t4 - llb);
+                bpS[(size_t)b * kLane + z] = bp;
+                tau0S[(size_t)b * kLane + z] = tau01.x;
+                // centerComp(b - 1)
+                const float factor = nj / bpr;
+                if (b > 0) facS[(size_t)(b - 1) * kLane + z] = factor;
+                const float2 fac = f2(factor), bpp = f2(before), bpc = f2(bp), xp = f2(xBefore), x2 = f2(x);
+                float2 tmp1 = mulz2(bpp, tp01, nz), tmp2 = mulz2(bpc, tau01, nz);
+                ci01 = add2(ci01, mulz2(add2(tmp1, tmp2), fac, nz));
+                m01 = add2(m01, mulz2(add2(mulz2(tmp1, xp, nz), mulz2(tmp2, x2, nz)), fac, nz));
+                tmp1 = mulz2(bpp, tp23, nz);
+                tmp2 = mulz2(bpc, tau23, nz);
+                ci23 = add2(ci23, mulz2(add2(tmp1, tmp2), fac, nz));
+                m23 = add2(m23, mulz2(add2(mulz2(tmp1, xp, nz), mulz2(tmp2, x2, nz)), fac, nz));
+                const float s1 = mul_rn(before, tp4), s2 = mul_rn(bp, tau4);
+                ci4 = add_rn(ci4, mul_rn(add_rn(s1, s2), factor));
+                m4 = add_rn(m4, mul_rn(add_rn(mul_rn(s1, xBefore), mul_rn(s2, x)), factor));
+                tp01 = tau01;
+                tp23 = tau23;
+                tp4 = tau4;
+            }
+        }
+        for (; b <= kBins; ++b)
+        {
+            const float most = fmaxf(mul_rn(mul_rn(h.binSize, bp), 1.0009765625f), h.binProbMin);
+            if (__all_sync(warp, (x >= muMax) & (most <= mul_rn(probSum, 7.450580596923828e-9f)))) break;
+            const float before = bp;
+            bare();
+            probSum = add_rn(probSum, binProb(before));
+        }
+        if (kFull)
+        {
+            const float2 hb = f2(halfBin);
+            ci01 = mulz2(ci01, hb, nz);
+            ci23 = mulz2(ci23, hb, nz);
+            m01 = mulz2(m01, hb, nz);
+            m23 = mulz2(m23, hb, nz);
+            ci[0] = ci01.x; ci[1] = ci01.y; ci[2] = ci23.x; ci[3] = ci23.y; ci[4] = mul_rn(ci4, hb.x);
+            mom1[0] = m01.x; mom1[1] = m01.y; mom1[2] = m23.x; mom1[3] = m23.y; mom1[4] = mul_rn(m4, hb.x);
+        }
+        ll = wps - mul_rn(h.nSum, hw_logf(probSum));
+    }
+    else
+    {
+        EmStepIo io;
+        io.h = h;
+        io.v = v;
+        io.bpS = bpS;
+        io.tau0S = tau0S;
+        io.facS = facS;
+        io.halfLog2pi = halfLog2pi;
+        io.negZero = k.negZero;
+        EmEStepGeneric<kFull>(io);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) { ci[i] = io.ci[i]; mom1[i] = io.mom1[i]; varinv[i] = io.varinv[i]; }
+        ll = io.ll;
+        safeOut = io.safe;
+    }
     const float ds = v.s - r.sExpect;
-    ll = ll - mul_rn(mul_rn(0.5f, mul_rn(ds, ds)), r.sExpectW);
-    safeOut = safe;
-    return ll;
+    return ll - mul_rn(mul_rn(0.5f, mul_rn(ds, ds)), r.sExpectW);
 }
 
 // One M-step (DmeEmHost.cpp:494-565) from the E-step's sums; ci is floored in
@@ -536,7 +743,7 @@ __device__ __forceinline__ void EmMStep(const KParams& k, const EmHist& h, const
     for (int a = 0; a < kAnalogs; ++a) v.mu[a + 1] = mul_rn(sv, k.relAmp[a]);
     // Background variance: second pass over the bins.  The scratch values of
     // boundary j + 1 are those of boundary j in the next bin, so each is
-    // loaded once, one bin ahead of its use.  Scratch slots of boundaries next
+    // loaded once.  Scratch slots of boundaries next
     // to empty bins hold stale values; they are loaded but only used for
     // occupied bins (or when !safe, where every boundary was written).
     // Bins that are empty for every ZMW of the warp add +0 to every sum (see
@@ -548,30 +755,44 @@ __device__ __forceinline__ void EmMStep(const KParams& k, const EmHist& h, const
         const int j0 = narrow ? h.wLo : 0;
         const int j1 = narrow ? h.wHi + 1 : kBins;
         float bpj = 0.0f, t0j = 0.0f;
-        uint32_t nj = 0u;
         if (j0 < j1)
         {
             bpj = bpS[(size_t)j0 * kLane + z];
             t0j = tau0S[(size_t)j0 * kLane + z];
-            nj = h.Count(j0);
         }
-        for (int j = j0; j < j1; ++j)
+        // four bins' values are loaded together (memory latency bounds this
+        // pass); past the last bin the last one's are loaded and not used
+        constexpr int kB = 4;
+        float jf = (float)j0;
+        for (int jj = j0; jj < j1; jj += kB)
         {
-            const float bpk = bpS[(size_t)(j + 1) * kLane + z], t0k = tau0S[(size_t)(j + 1) * kLane + z];
-            const float fj = facS[(size_t)j * kLane + z];
-            const uint32_t nk = (j + 1 < kBins) ? h.Count(j + 1) : 0u;
-            if (!safe || nj != 0u)      // an empty bin adds +0 (see the E-step)
+            float bpk[kB], t0k[kB], fj[kB];
+            uint32_t nj[kB];
+#pragma unroll
+            for (int q = 0; q < kB; ++q)
             {
-                const float xj = h.BinStart(j) - v.mu[0];
-                const float xk = h.BinStart(j + 1) - v.mu[0];
-                float tmp = mul_rn(mul_rn(mul_rn(bpj, xj), xj), t0j);
-                tmp = add_rn(tmp, mul_rn(mul_rn(mul_rn(bpk, xk), xk), t0k));
-                tmp = mul_rn(tmp, fj);
-                mom2 = add_rn(mom2, tmp);
+                const int j = jj + q < j1 ? jj + q : j1 - 1;
+                bpk[q] = bpS[(size_t)(j + 1) * kLane + z];
+                t0k[q] = tau0S[(size_t)(j + 1) * kLane + z];
+                fj[q] = facS[(size_t)j * kLane + z];
+                nj[q] = h.Count(j);
             }
-            bpj = bpk;
-            t0j = t0k;
-            nj = nk;
+#pragma unroll
+            for (int q = 0; q < kB; ++q)
+            {
+                if (jj + q < j1 && (!safe || nj[q] != 0u))      // an empty bin adds +0 (see the E-step)
+                {
+                    const float xj = add_rn(h.lb, mul_rn(jf, h.binSize)) - v.mu[0];
+                    const float xk = add_rn(h.lb, mul_rn(jf + 1.0f, h.binSize)) - v.mu[0];
+                    float tmp = mul_rn(mul_rn(mul_rn(bpj, xj), xj), t0j);
+                    tmp = add_rn(tmp, mul_rn(mul_rn(mul_rn(bpk[q], xk), xk), t0k[q]));
+                    tmp = mul_rn(tmp, fj[q]);
+                    mom2 = add_rn(mom2, tmp);
+                }
+                jf += 1.0f;
+                bpj = bpk[q];
+                t0j = t0k[q];
+            }
         }
     }
     mom2 = mul_rn(mom2, mul_rn(0.5f, h.binSize));
@@ -622,7 +843,7 @@ __device__ __forceinline__ int ChooseStart(const KParams& k, const EmHist& h, co
 // reference-start variant carries neither the start choice's values nor the
 // clock's counters through its EM loop (they cost registers there).
 template <bool Mapped, bool Learned, bool Clock>
-__global__ void __launch_bounds__(kLane, 10) DmeEstimateKernel(DmeArgs A, KParams k)
+__global__ void __launch_bounds__(kLane, 8) DmeEstimateKernel(DmeArgs A, KParams k)
 {
     LaneMap map = A.map;
     if (!Mapped) map.list = nullptr;      // the single-pool variant compiles without the lane list
@@ -938,7 +1159,7 @@ __device__ __forceinline__ float EmStep(const EmVars& a, const EmVars& b)
     return d;
 }
 
-__global__ void __launch_bounds__(kLane, 12) DmeEmFitKernel(DmeFitArgs A, KParams k)
+__global__ void __launch_bounds__(kLane, 8) DmeEmFitKernel(DmeFitArgs A, KParams k)
 {
     const int l = blockIdx.x;
     const int z = threadIdx.x;

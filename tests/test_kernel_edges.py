@@ -35,6 +35,51 @@ def _both(cfg, lanes, F, call):
         _eq(f"output {i}", a, b)
 
 
+def _estimate_inputs(lanes):
+    """Histogram, statistics and prior of a pool's first estimate (oracle)."""
+    cfg = workloads.small_config()
+    tr = synth.traces(lanes, 512 * 8, seed=5, gain_sigma=0.3, empty_fraction=0.2)
+    pipe = harness.Pipeline(harness.OracleBackend(cfg, lanes, 512), cfg)
+    for c in range(8):
+        rec = pipe.process(np.ascontiguousarray(tr[:, c * 512:(c + 1) * 512]), c * 512)
+        if "init_models" in rec:
+            prior = rec["init_models"]
+        if "hist" in rec:
+            return cfg, rec["hist"], rec["agg"], prior
+    raise AssertionError("no estimate")
+
+
+@pytest.mark.parametrize("kind", ["plain", "one_bin", "ends", "far", "empty", "narrow", "inf_mean", "zero_var",
+                                  "wide_bins", "bright"])
+def test_estimate_paths(kind):
+    lanes = 2
+    cfg, hist, stats, prior = _estimate_inputs(lanes)
+    hist, stats, prior = hist.copy(), stats.copy(), prior.copy()
+    odd = slice(None, None, 3)          # ZMWs of every warp, not all of them
+    bins = hist["bin_count"]
+    if kind == "one_bin":
+        bins[:, :, odd] = 0
+        bins[:, 40, odd] = 4000
+    elif kind == "ends":
+        bins[:, 0, odd] = 7
+        bins[:, 299, odd] = 5
+    elif kind == "far":
+        bins[:, 250:260, 5] = 1
+    elif kind == "empty":
+        bins[:, :, odd] = 0
+    elif kind == "narrow":
+        hist["bin_size"][:, odd] *= np.float32(1e-3)
+    elif kind == "inf_mean":
+        prior["analogs"]["means"][:, 1, odd] = 0x7c00
+    elif kind == "zero_var":
+        stats["baseline_stats"]["moment2"][:, odd] = 0.0
+    elif kind == "wide_bins":
+        hist["bin_size"][:, odd] *= np.float32(1e5)
+    elif kind == "bright":
+        prior["analogs"]["means"][:, :, odd] = abi.f32_to_f16(np.float32(6.0e4))
+    _both(cfg, lanes, 512, lambda b: b.estimate(hist, stats, (0, 4096), (0, 512), prior))
+
+
 @pytest.mark.parametrize("F", [48, 512])
 @pytest.mark.parametrize("pedestal,sensitivity,extreme", [(0, 1.0, False), (13, 1.9, False), (-32768, 0.01, True),
                                                           (32767, 62.0, True), (5, 100.0, True), (0, 3.0e7, False)])
