@@ -301,13 +301,25 @@ struct KParams
     uint8_t analogMap[kAnalogs];
     // -0.0f, read at run time by the packed products (mulz2)
     float negZero;
-    // labeler, 9-way rows 0, 5, 6, 7, 8 (index 0..4): the transition
-    // constants (T[R][5], T[R][9]) of the source groups 5..8 and 9..12, and
+    // labeler, 9-way rows 0, 5, 6, 7, 8: source groups 5..8 (A) and 9..12 (B);
     // whether every such row's constants are equal within each group (then
     // the rows take the grouped arg-max)
-    float2 grp9[5];
+    // whether every such row's constants are equal within each group and every
+    // constant is finite (then the labeler takes the grouped step); the
+    // grouped step's constants follow, as the pairs it adds: the baseline
+    // row's (t_0, t_A, t_B), rows 5/6 and 7/8 of the pulse-up states, and the
+    // two-way rows 1/2, 3/4 (full) and 9/10, 11/12 (down) with their first and
+    // second source; grpTol bounds the 9-way constants' share of the rounding
+    // margin (see GroupedStep in labeler.cu)
     int grouped9;
+    float grpRow0[3];
+    float grpTol;
+    float2 grpUp0[2], grpUpA[2], grpUpB[2];
+    float2 grpTwo[4][2];
 };
+
+// The grouped step's rounding margin is this times the magnitudes it adds.
+constexpr float kGrpTol = 4.76837158203125e-07f;       // 2^-21
 
 inline void FillParams(const hw_config& cfg, const hwp::Derived& d, KParams* k)
 {
@@ -341,17 +353,37 @@ inline void FillParams(const hw_config& cfg, const hwp::Derived& d, KParams* k)
     k->roiUpper = cfg.roi_upper_threshold; k->roiLower = cfg.roi_lower_threshold;
     k->ampThresh = d.ampThresh; k->widthThresh = d.widthThresh; k->maxCalls = (int)cfg.max_calls_per_zmw;
     k->negZero = -0.0f;
-    // Grouped 9-way rows: bitwise-equal, non-NaN constants within each group.
+    // Grouped 9-way rows: bitwise-equal constants within each group.
     const int rows9[5] = {0, 5, 6, 7, 8};
     bool grouped = true;
+    float tMax = 0.0f;
     for (int i = 0; i < 5; ++i)
     {
         const float* t = d.trans[rows9[i]];
-        k->grp9[i] = make_float2(t[5], t[9]);
         for (int g = 5; g <= 9; g += 4)
-            for (int s = g; s < g + 4; ++s)
-                grouped &= (t[s] == t[s]) && std::memcmp(&t[s], &t[g], sizeof(float)) == 0;
-        grouped &= (t[0] == t[0]);
+            for (int s = g; s < g + 4; ++s) grouped &= std::memcmp(&t[s], &t[g], sizeof(float)) == 0;
+        for (int c : {0, 5, 9}) tMax = std::max(tMax, std::fabs(t[c]));
+    }
+    for (int r = 0; r < kStates; ++r)
+        for (int c = 0; c < kStates; ++c)
+        {
+            const bool used = (r == 0 || (r >= 5 && r <= 8)) ? (c == 0 || c >= 5)
+                              : r <= 4                       ? (c == r || c == r + 4)
+                                                             : (c == r - 8 || c == r - 4);
+            if (used) grouped &= std::isfinite(d.trans[r][c]);
+        }
+    k->grpTol = tMax * kGrpTol;
+    k->grpRow0[0] = d.trans[0][0]; k->grpRow0[1] = d.trans[0][5]; k->grpRow0[2] = d.trans[0][9];
+    for (int q = 0; q < 2; ++q)
+    {
+        const int r = 5 + 2 * q, u = 1 + 2 * q, w = 9 + 2 * q;
+        k->grpUp0[q] = make_float2(d.trans[r][0], d.trans[r + 1][0]);
+        k->grpUpA[q] = make_float2(d.trans[r][5], d.trans[r + 1][5]);
+        k->grpUpB[q] = make_float2(d.trans[r][9], d.trans[r + 1][9]);
+        k->grpTwo[q][0] = make_float2(d.trans[u][u], d.trans[u + 1][u + 1]);
+        k->grpTwo[q][1] = make_float2(d.trans[u][u + 4], d.trans[u + 1][u + 5]);
+        k->grpTwo[2 + q][0] = make_float2(d.trans[w][w - 8], d.trans[w + 1][w - 7]);
+        k->grpTwo[2 + q][1] = make_float2(d.trans[w][w - 4], d.trans[w + 1][w - 3]);
     }
     k->grouped9 = grouped ? 1 : 0;
 }

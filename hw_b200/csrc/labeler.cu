@@ -4,9 +4,9 @@
 // TA/RoiHost.h:75-249 (TA = src/basecaller/basecaller/traceAnalysis).
 //
 // One thread per ZMW.  Per chunk a thread
-//   1. runs the ROI forward recursion over the 24 latent frames and the chunk,
-//      keeping the 2-bit ROI codes packed 16 per word in local memory, then
-//      the backward recursion (1 bit per frame);
+//   1. gathers the ROI's two threshold bits of the 24 latent frames and the
+//      chunk, 32 frames a word, and runs the forward and backward recursions
+//      on whole words;
 //   2. runs the max-plus Viterbi over 24 latent + F-8 chunk frames + 16
 //      look-ahead frames in fp32 with the reference's operation order and
 //      tie rule (a later source state wins ties);
@@ -26,13 +26,15 @@ namespace hwk {
 // reference's operation order (see the f32x2 helpers); constants the
 // reference recomputes per frame from per-ZMW values (-0.5 times the inverse
 // variances, the negated caps, means and log means, the dimmest analog's
-// fallback condition) are formed once in Setup, with the same roundings.
+// fallback condition) are formed once in Setup, with the same roundings
+// (halving is exact, so (-0.5 y) / var is y times -0.5 / var).
 struct ZScorer
 {
-    float bgMean, bInvVar, bgFixed, x0, nhBInv;
-    float2 negMean[2], pInv[2], ffFixed[2], nhPInv[2], negX1[2], negLogP[2], x1[2];
+    float bgMean, bgFixed, x0, nhBInv;
+    float2 negMean[2], ffFixed[2], nhPInv[2], negX1[2], negLogP[2];
     float fbMean, fbNormTerm, fbScale;
     bool fbUse;     // x0 > x1 of the dimmest analog: its up/down score is the normal fallback
+    bool ordinary;  // every constant finite: no score of an int16 trace value is NaN or infinite
 
     __device__ __forceinline__ void Setup(const KParams& k, const hw_lane_model& m, int z)
     {
@@ -42,9 +44,8 @@ struct ZScorer
         const float bVar = h2f(m.baseline.vars[z]);
         const float bSigma = sqrtf(bVar);
         x0 = add_rn(bMean, mul_rn(bSigma, k.sqrtHalfPi));
-        bInvVar = 1.0f / bVar;
-        nhBInv = mul_rn(nhalf, bInvVar);
-        float aM[kAnalogs], pI[kAnalogs], fx[kAnalogs], lp[kAnalogs], xx[kAnalogs];
+        nhBInv = mul_rn(nhalf, 1.0f / bVar);
+        float aM[kAnalogs], nh[kAnalogs], fx[kAnalogs], lp[kAnalogs], xx[kAnalogs];
 #pragma unroll
         for (int a = 0; a < kAnalogs; ++a)
         {
@@ -53,7 +54,7 @@ struct ZScorer
             const float aVar = h2f(m.analogs[a].vars[z]);
             const float aSigma = sqrtf(aVar);
             xx[a] = aMean - mul_rn(aSigma, k.sqrtHalfPi);
-            pI[a] = 1.0f / aVar;
+            nh[a] = mul_rn(nhalf, 1.0f / aVar);
             fx[a] = mul_rn(nhalf, hw_logf(aVar)) - log2pi_f / 2.0f;
             aM[a] = aMean;
         }
@@ -62,11 +63,9 @@ struct ZScorer
         {
             const int a = 2 * q;
             negMean[q] = f2(-aM[a], -aM[a + 1]);
-            pInv[q] = f2(pI[a], pI[a + 1]);
             ffFixed[q] = f2(fx[a], fx[a + 1]);
-            nhPInv[q] = f2(mul_rn(nhalf, pI[a]), mul_rn(nhalf, pI[a + 1]));
+            nhPInv[q] = f2(nh[a], nh[a + 1]);
             negX1[q] = f2(-xx[a], -xx[a + 1]);
-            x1[q] = f2(xx[a], xx[a + 1]);
             negLogP[q] = f2(-lp[a], -lp[a + 1]);
         }
         {
@@ -83,15 +82,24 @@ struct ZScorer
         fbUse = !(x0 <= xx[3]);
         bgFixed = mul_rn(nhalf, hw_logf(bVar)) - log2pi_f / 2.0f;
         bgMean = bMean;
+        ordinary = isfinite(bgMean) & isfinite(bgFixed) & isfinite(x0) & isfinite(nhBInv) & isfinite(fbMean) &
+                   isfinite(fbNormTerm) & isfinite(fbScale);
+#pragma unroll
+        for (int a = 0; a < kAnalogs; ++a)
+            ordinary &= isfinite(aM[a]) & isfinite(nh[a]) & isfinite(fx[a]) & isfinite(lp[a]) & isfinite(xx[a]);
     }
 
-    // StateScores for states 0..8 (states 9..12 repeat 5..8).
+    __device__ __forceinline__ float Background(float data) const
+    {
+        const float y = data - bgMean;
+        return add_rn(mul_rn(mul_rn(y, nhBInv), y), bgFixed);
+    }
+
+    // StateScores for states 0..8 (states 9..12 repeat 5..8), for constants
+    // and a trace value of any kind.
     __device__ __forceinline__ void Scores(float data, float* out, float2 nz) const
     {
-        {
-            const float y = data - bgMean;
-            out[0] = add_rn(mul_rn(mul_rn(mul_rn(-0.5f, y), bInvVar), y), bgFixed);
-        }
+        out[0] = Background(data);
         const float2 d2 = f2(data);
         const bool low = data < x0;
 #pragma unroll
@@ -99,13 +107,13 @@ struct ZScorer
         {
             // full frame: ((-0.5 y) / var) y + fixed, y = data - mean
             const float2 y = add2(d2, negMean[q]);
-            const float2 full = add2(mulz2(mul2(mul2(f2(-0.5f), y), pInv[q]), y, nz), ffFixed[q]);
+            const float2 full = add2(mulz2(mul2(y, nhPInv[q]), y, nz), ffFixed[q]);
             // sub-frame Gauss cap: (extrema ? (-0.5 / var) dv^2 : 0) - log(mean - baseline mean)
             const float2 negCap = low ? f2(-x0) : negX1[q];
             const float2 fixedTerm = low ? f2(nhBInv) : nhPInv[q];
             const float2 dv = add2(d2, negCap);
             const float2 prod = mulz2(fixedTerm, mul2(dv, dv), nz);
-            const bool ex = low | (data > x1[q].x), ey = low | (data > x1[q].y);
+            const bool ex = low | (data > -negX1[q].x), ey = low | (data > -negX1[q].y);
             float2 sub = add2(f2(ex ? prod.x : 0.0f, ey ? prod.y : 0.0f), negLogP[q]);
             if (q == 1 && fbUse)
             {
@@ -120,6 +128,41 @@ struct ZScorer
             out[2 + 2 * q] = full.y;
             out[5 + 2 * q] = sub.x;
             out[6 + 2 * q] = sub.y;
+        }
+    }
+
+    // The same scores for `ordinary` constants, as the pairs of analogs 0/1
+    // and 2/3.  With nothing NaN the clamps are plain minima; the cap's
+    // "extrema" selection is a maximum with 0 (its square term is then -0,
+    // which changes no sum); the baseline side of the cap does not depend on
+    // the analog.
+    __device__ __forceinline__ void OrdinaryScores(float data, float& s0, float2 (&fullS)[2], float2 (&subS)[2],
+                                                   float2 nz) const
+    {
+        s0 = Background(data);
+        const float2 d2 = f2(data);
+        const bool low = data < x0;
+        const float dl = data - x0;
+        const float lowProd = mul_rn(nhBInv, mul_rn(dl, dl));
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+        {
+            const float2 y = add2(d2, negMean[q]);
+            const float2 full = add2(mulz2(mul2(y, nhPInv[q]), y, nz), ffFixed[q]);
+            float2 dv = add2(d2, negX1[q]);
+            dv = f2(fmaxf(dv.x, 0.0f), fmaxf(dv.y, 0.0f));
+            const float2 prod = mulz2(nhPInv[q], mul2(dv, dv), nz);
+            float2 sub = add2(f2(low ? lowProd : prod.x, low ? lowProd : prod.y), negLogP[q]);
+            if (q == 1)
+            {
+                const float dm = data - fbMean;
+                const float fb = fbNormTerm - mul_rn(mul_rn(dm, dm), fbScale);
+                sub.y = fbUse ? fb : sub.y;
+            }
+            const float2 fm1 = add2(full, f2(-1.0f));
+            const float cx = min3(sub.x, fm1.x, 0.0f), cy = min3(sub.y, fm1.y, 0.0f);
+            fullS[q] = full;
+            subS[q] = f2(y.x > 0.0f ? cx : sub.x, y.y > 0.0f ? cy : sub.y);
         }
     }
 };
@@ -186,58 +229,6 @@ __device__ __forceinline__ float NineWayRow(const KParams& k, float score, const
     return mv;
 }
 
-// Grouped 9-way rows.  When a row's transition constants are equal within
-// each source group (t_A for states 5..8, t_B for 9..12; KParams::grouped9),
-// its candidates of group G are RN(a_G + ll[s]) with a_G = RN(score + t_G)
-// the same for the whole group, and RN(a_G + x) is monotone in x.  So the
-// group's best value is RN(a_G + m_G), m_G the group's largest ll, reached
-// by the last state holding m_G, unless a later state of the group rounds
-// to the same sum: that needs RN(a_G + m'_G) == RN(a_G + m_G), m'_G the
-// largest ll after that state, and sends the frame to the generic rows.  m_G,
-// its last position and m'_G are shared by the five 9-way rows of a frame.
-struct GroupMax
-{
-    float m;        // largest ll of the group
-    float after;    // largest ll after its last position (NaN: none)
-    uint32_t pos;   // last position of m, 0..3
-};
-
-// Right to left with strict comparisons: the last position of the maximum.
-__device__ __forceinline__ GroupMax ScanGroup(float2 lo, float2 hi)
-{
-    GroupMax g{hi.y, __int_as_float(0x7fffffff), 3u};
-    auto step = [&](float v, uint32_t p) {
-        const bool gt = v > g.m;
-        g.after = gt ? g.m : g.after;
-        g.m = gt ? v : g.m;
-        g.pos = gt ? p : g.pos;
-    };
-    step(hi.x, 2u);
-    step(lo.y, 1u);
-    step(lo.x, 0u);
-    return g;
-}
-
-// One grouped 9-way row (index i of rows 0, 5, 6, 7, 8): returns the row's
-// value; base receives the winner's code (0 for state 0, s - 4 for s in
-// 5..12) unshifted; slow is set when the group winner is not certain.
-template <int i>
-__device__ __forceinline__ float GroupedRow(const KParams& k, float score, float ll0, float2 gm, float2 gafter,
-                                            uint32_t codeA, uint32_t codeB, uint32_t& base, bool& slow)
-{
-    constexpr int R = (i == 0) ? 0 : i + 4;
-    const float c0 = add_rn(add_rn(score, k.trans[R][0]), ll0);
-    const float2 a = add2(f2(score), k.grp9[i]);
-    const float2 gv = add2(a, gm);          // the groups' best candidates
-    const float2 nv = add2(a, gafter);      // the best after each group's winner
-    const bool geA = gv.x >= c0;
-    const float mv = geA ? gv.x : c0;
-    const bool geB = gv.y >= mv;
-    base = geB ? codeB : (geA ? codeA : 0u);
-    slow |= geB ? (nv.y == gv.y) : (geA & (nv.x == gv.x));
-    return geB ? gv.y : mv;
-}
-
 // Two 2-way rows, R and R + 1, with scores s.x, s.y: their first sources are
 // the pair qa, their second the pair qb.
 template <int R, int qa, int qb, bool Margin>
@@ -261,72 +252,35 @@ __device__ __forceinline__ float2 TwoWayRows(const KParams& k, float2 s, const S
     return f2(gx ? second.x : first.x, gy ? second.y : first.y);
 }
 
-// One Viterbi recursion step; returns the packed traceback word.  With
-// Margin, gap[r] receives row r's decision gap.
-template <bool Margin = false, bool Grouped = false>
-__device__ __forceinline__ uint32_t ViterbiStep(const KParams& k, const ZScorer& sc, float data, bool isRoi,
+// One Viterbi recursion step over the generic rows; returns the packed
+// traceback word.  With Margin, gap[r] receives row r's decision gap.
+template <bool Margin>
+__device__ __forceinline__ uint32_t ViterbiStep(const KParams& k, const ZScorer& sc, float data, float npen,
                                                 StateLL& ll, float* gap = nullptr)
 {
-    static_assert(!(Margin && Grouped), "margins come from the generic rows");
     float sco[9];
     sc.Scores(data, sco, f2(k.negZero));
     uint32_t cd[9];
     float gl[kStates];
-    float n0, n5, n6, n7, n8;
-    if constexpr (Grouped)
-    {
-        const GroupMax gA = ScanGroup(ll.p[2], ll.p[3]), gB = ScanGroup(ll.p[4], ll.p[5]);
-        const float2 gm = f2(gA.m, gB.m), ga = f2(gA.after, gB.after);
-        const uint32_t codeA = 1u + gA.pos, codeB = 5u + gB.pos;
-        // a NaN among the rows' inputs (or an inf - inf) takes the generic rows
-        const float2 lsum = add2(add2(ll.p[2], ll.p[3]), add2(ll.p[4], ll.p[5]));
-        const float ssum = add_rn(add_rn(add_rn(sco[0], sco[5]), add_rn(sco[6], sco[7])), sco[8]);
-        bool slow = isnan(add_rn(add_rn(lsum.x, lsum.y), add_rn(ll.s0, ssum)));
-        uint32_t b0, b5, b6, b7, b8;
-        n0 = GroupedRow<0>(k, sco[0], ll.s0, gm, ga, codeA, codeB, b0, slow);
-        n5 = GroupedRow<1>(k, sco[5], ll.s0, gm, ga, codeA, codeB, b5, slow);
-        n6 = GroupedRow<2>(k, sco[6], ll.s0, gm, ga, codeA, codeB, b6, slow);
-        n7 = GroupedRow<3>(k, sco[7], ll.s0, gm, ga, codeA, codeB, b7, slow);
-        n8 = GroupedRow<4>(k, sco[8], ll.s0, gm, ga, codeA, codeB, b8, slow);
-        if (slow)
-        {
-            n0 = NineWayRow<0, false>(k, sco[0], ll, cd[0], gl[0]);
-            n5 = NineWayRow<5, false>(k, sco[5], ll, cd[1], gl[5]);
-            n6 = NineWayRow<6, false>(k, sco[6], ll, cd[2], gl[6]);
-            n7 = NineWayRow<7, false>(k, sco[7], ll, cd[3], gl[7]);
-            n8 = NineWayRow<8, false>(k, sco[8], ll, cd[4], gl[8]);
-        }
-        else
-        {
-            cd[0] = b0;
-            cd[1] = b5 << 4;
-            cd[2] = b6 << 8;
-            cd[3] = b7 << 12;
-            cd[4] = b8 << 16;
-        }
-    }
-    else
-    {
-        n0 = NineWayRow<0, Margin>(k, sco[0], ll, cd[0], gl[0]);
-        n5 = NineWayRow<5, Margin>(k, sco[5], ll, cd[1], gl[5]);
-        n6 = NineWayRow<6, Margin>(k, sco[6], ll, cd[2], gl[6]);
-        n7 = NineWayRow<7, Margin>(k, sco[7], ll, cd[3], gl[7]);
-        n8 = NineWayRow<8, Margin>(k, sco[8], ll, cd[4], gl[8]);
-    }
+    const float n0 = NineWayRow<0, Margin>(k, sco[0], ll, cd[0], gl[0]);
+    const float n5 = NineWayRow<5, Margin>(k, sco[5], ll, cd[1], gl[5]);
+    const float n6 = NineWayRow<6, Margin>(k, sco[6], ll, cd[2], gl[6]);
+    const float n7 = NineWayRow<7, Margin>(k, sco[7], ll, cd[3], gl[7]);
+    const float n8 = NineWayRow<8, Margin>(k, sco[8], ll, cd[4], gl[8]);
     // full rows: (r, r + 4); down rows: (r - 8, r - 4)
     const float2 n12 = TwoWayRows<1, 0, 2, Margin>(k, f2(sco[1], sco[2]), ll, cd[5], gl[1], gl[2]);
     const float2 n34 = TwoWayRows<3, 1, 3, Margin>(k, f2(sco[3], sco[4]), ll, cd[6], gl[3], gl[4]);
     const float2 n9a = TwoWayRows<9, 0, 2, Margin>(k, f2(sco[5], sco[6]), ll, cd[7], gl[9], gl[10]);
     const float2 nbc = TwoWayRows<11, 1, 3, Margin>(k, f2(sco[7], sco[8]), ll, cd[8], gl[11], gl[12]);
     // non-ROI frames: every state but the baseline gets -inf (x - inf)
-    const float2 npen = f2(isRoi ? -0.0f : -__int_as_float(0x7f800000));
+    const float2 pen = f2(npen);
     ll.s0 = n0;
-    ll.p[0] = add2(n12, npen);
-    ll.p[1] = add2(n34, npen);
-    ll.p[2] = add2(f2(n5, n6), npen);
-    ll.p[3] = add2(f2(n7, n8), npen);
-    ll.p[4] = add2(n9a, npen);
-    ll.p[5] = add2(nbc, npen);
+    ll.p[0] = add2(n12, pen);
+    ll.p[1] = add2(n34, pen);
+    ll.p[2] = add2(f2(n5, n6), pen);
+    ll.p[3] = add2(f2(n7, n8), pen);
+    ll.p[4] = add2(n9a, pen);
+    ll.p[5] = add2(nbc, pen);
     if constexpr (Margin)
     {
 #pragma unroll
@@ -335,8 +289,129 @@ __device__ __forceinline__ uint32_t ViterbiStep(const KParams& k, const ZScorer&
     return ((cd[0] | cd[1] | cd[2]) | (cd[3] | cd[4])) | ((cd[5] | cd[6]) | (cd[7] | cd[8]));
 }
 
-// Source state of `state` recorded in traceback word `w`.
-__device__ __forceinline__ int TraceSource(uint32_t w, int state)
+// acc shifted left by n with the top n bits of v: n = 1 appends v's sign.
+template <int n> __device__ __forceinline__ uint32_t PushTop(uint32_t acc, float v)
+{
+    return __funnelshift_l(__float_as_uint(v), acc, n);
+}
+// b - a of both components, rounded once (the product by -1 is exact).
+__device__ __forceinline__ float2 sub2(float2 b, float2 a) { return fma2(a, f2(-1.0f), b); }
+
+// Traceback word of a grouped step that took the generic rows: their word
+// shifted by kGenericShift, with kGenericWord set.
+constexpr uint32_t kGenericWord = 4u;
+constexpr int kGenericShift = 3;
+
+// The step when the 9-way rows' transition constants are equal within each
+// source group (t_A for states 5..8, t_B for 9..12; KParams::grouped9).
+//
+// A row's candidates of group G are RN(a_G + ll[s]) with a_G = RN(score + t_G)
+// the same for the whole group, and RN(a_G + x) is monotone in x: the group's
+// best candidate is RN(a_G + m_G), m_G the group's largest ll.  It belongs to
+// the last state holding m_G unless another state's sum rounds to the same
+// value, which needs their ll to differ by no more than 2^-22 |a_G + m_G|.  So
+// m_G and its position are found once for the five rows, by two rounds of
+// pairwise comparisons, and a frame where one of a group's comparisons is
+// closer than 2^-21 (|score| + |t| + |m_G|) over all rows, or whose scorer is
+// not `ordinary`, takes the generic rows.
+//
+// Every decision "the later candidate is at least the earlier one" is the sign
+// of their difference: 0 for yes (also for equal values and for two -inf,
+// whose difference is the positive quiet NaN; ll never holds -0 or +inf).  So
+// a value needs one maximum and a decision one subtraction (FMA pipe) and one
+// funnel shift that appends the sign to the traceback word: with compares and
+// selects instead (422 thread instructions a ZMW-frame over the kernel, 68% of
+// the ALU pipe) 4096 lanes x 512 frames took 2145 us; now 299, 55% and 1560 us.
+// Issue and ALU latency bound it now (65% of issue slots at 5 warps a
+// scheduler, the most that 96 registers allow; 4 and 6 warps measured 1659 and
+// 1616 us).
+//
+// Word: bit 2 s + 1 of state s is its last decision (0: the later of two
+// sources, or group B), bit 2 s of a 9-way state the decision before it (0:
+// group A, 1: state 0); bits 31..29 and 28..26 hold the comparisons of groups A
+// and B: 6 against 5, 8 against 7 and the second against the first pair
+// (likewise 9..12).  Bit 2 is kGenericWord.
+__device__ __forceinline__ uint32_t GroupedStep(const KParams& k, const ZScorer& sc, float data, float npen, bool bad,
+                                                StateLL& ll)
+{
+    const float2 nz = f2(k.negZero);
+    float s0;
+    float2 full[2], sub[2];
+    sc.OrdinaryScores(data, s0, full, sub, nz);
+    const float hA1 = fmaxf(ll.p[2].x, ll.p[2].y), hA2 = fmaxf(ll.p[3].x, ll.p[3].y), mA = fmaxf(hA1, hA2);
+    const float hB1 = fmaxf(ll.p[4].x, ll.p[4].y), hB2 = fmaxf(ll.p[5].x, ll.p[5].y), mB = fmaxf(hB1, hB2);
+    const float eA1 = ll.p[2].y - ll.p[2].x, eA2 = ll.p[3].y - ll.p[3].x, eA3 = hA2 - hA1;
+    const float eB1 = ll.p[4].y - ll.p[4].x, eB2 = ll.p[5].y - ll.p[5].x, eB3 = hB2 - hB1;
+    // an empty group (all -inf) has NaN differences: not slow
+    const float sMax = max3(max3(fabsf(s0), fabsf(sub[0].x), fabsf(sub[0].y)), fabsf(sub[1].x), fabsf(sub[1].y));
+    const float tol = fma_rn(sMax, kGrpTol, k.grpTol);
+    const bool slow = bad | (min3(fabsf(eA1), fabsf(eA2), fabsf(eA3)) <= fma_rn(fabsf(mA), kGrpTol, tol)) |
+                      (min3(fabsf(eB1), fabsf(eB2), fabsf(eB3)) <= fma_rn(fabsf(mB), kGrpTol, tol));
+    if (slow) return (ViterbiStep<false>(k, sc, data, npen, ll) << kGenericShift) | kGenericWord;
+
+    uint32_t hi = PushTop<1>(0u, eA1);
+    hi = PushTop<1>(hi, eA2);
+    hi = PushTop<1>(hi, eA3);
+    hi = PushTop<1>(hi, eB1);
+    hi = PushTop<1>(hi, eB2);
+    hi = PushTop<1>(hi, eB3);
+    const float2 l0 = f2(ll.s0), gA = f2(mA), gB = f2(mB);
+    float2 dUA[2], dUB[2], dF[2], dD[2], nU[2], nF[2], nD[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+    {
+        const float2 c0 = add2(add2(sub[q], k.grpUp0[q]), l0);
+        const float2 cA = add2(add2(sub[q], k.grpUpA[q]), gA);
+        const float2 cB = add2(add2(sub[q], k.grpUpB[q]), gB);
+        nU[q] = f2(max3(c0.x, cA.x, cB.x), max3(c0.y, cA.y, cB.y));
+        dUA[q] = sub2(cA, c0);
+        dUB[q] = sub2(cB, nU[q]);
+        const float2 f1 = add2(add2(full[q], k.grpTwo[q][0]), ll.p[q]);
+        const float2 f2_ = add2(add2(full[q], k.grpTwo[q][1]), ll.p[2 + q]);
+        nF[q] = f2(fmaxf(f1.x, f2_.x), fmaxf(f1.y, f2_.y));
+        dF[q] = sub2(f2_, f1);
+        const float2 d1 = add2(add2(sub[q], k.grpTwo[2 + q][0]), ll.p[q]);
+        const float2 d2 = add2(add2(sub[q], k.grpTwo[2 + q][1]), ll.p[2 + q]);
+        nD[q] = f2(fmaxf(d1.x, d2.x), fmaxf(d1.y, d2.y));
+        dD[q] = sub2(d2, d1);
+    }
+    const float c0 = add_rn(add_rn(s0, k.grpRow0[0]), ll.s0);
+    const float cA = add_rn(add_rn(s0, k.grpRow0[1]), mA);
+    const float cB = add_rn(add_rn(s0, k.grpRow0[2]), mB);
+    const float n0 = max3(c0, cA, cB);
+    hi = PushTop<2>(hi, dD[1].y);
+    hi = PushTop<2>(hi, dD[1].x);
+    hi = PushTop<2>(hi, dD[0].y);
+    hi = PushTop<2>(hi, dD[0].x);
+    hi = PushTop<1>(hi, dUB[1].y);
+    hi = PushTop<1>(hi, dUA[1].y);
+    uint32_t lo = PushTop<1>(0u, dUB[1].x);
+    lo = PushTop<1>(lo, dUA[1].x);
+    lo = PushTop<1>(lo, dUB[0].y);
+    lo = PushTop<1>(lo, dUA[0].y);
+    lo = PushTop<1>(lo, dUB[0].x);
+    lo = PushTop<1>(lo, dUA[0].x);
+    lo = PushTop<2>(lo, dF[1].y);
+    lo = PushTop<2>(lo, dF[1].x);
+    lo = PushTop<2>(lo, dF[0].y);
+    lo = PushTop<2>(lo, dF[0].x);
+    lo = PushTop<1>(lo, cB - n0);
+    lo = PushTop<1>(lo, cA - c0);
+    // non-ROI frames: every state but the baseline gets -inf (x - inf)
+    const float2 pen = f2(npen);
+    ll.s0 = n0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+    {
+        ll.p[q] = add2(nF[q], pen);
+        ll.p[2 + q] = add2(nU[q], pen);
+        ll.p[4 + q] = add2(nD[q], pen);
+    }
+    return __byte_perm(lo, hi, 0x5410) & ~kGenericWord;
+}
+
+// Source state of `state` recorded in a generic step's traceback word `w`.
+__device__ __forceinline__ int GenericSource(uint32_t w, int state)
 {
     if (state == 0 || state >= 5 && state <= 8)
     {
@@ -353,30 +428,89 @@ __device__ __forceinline__ int TraceSource(uint32_t w, int state)
     return b ? state - 4 : state - 8;
 }
 
+// Source state of `state` recorded in traceback word `w`.  The two-way rows of
+// an analog (full and down) choose between its full state (first) and its up
+// state; a 9-way row between state 0, the up state and the down state of its
+// group's largest ll, whose position (0..3) the group's three comparisons give
+// through a table of two bits an entry.
+template <bool Grouped> __device__ __forceinline__ int TraceSource(uint32_t w, int state)
+{
+    if (!Grouped) return GenericSource(w, state);
+    if (w & kGenericWord) return GenericSource(w >> kGenericShift, state);
+    const uint32_t v = w >> (2 * state);
+    const uint32_t first = (v >> 1) & 1u;              // not the last source (group)
+    const uint32_t nine = (0x1e1u >> state) & 1u;
+    const uint32_t pos = (0x2367u >> ((w >> (25u + 3u * first)) & 14u)) & 3u;
+    const uint32_t sub = nine ? pos : (uint32_t)(state + 3) & 3u;
+    const int src = (int)(5u + 4u * nine - 4u * first + sub);
+    return (nine & v) & first ? 0 : src;
+}
 
-// x / c, correctly rounded, for the ROI's constants c = sqrt(2) and sqrt(3):
-// q = x * RN(1/c) corrected once with the exact remainder x - q c (Markstein's
-// correction); zero and non-finite quotients pass through.  An exhaustive
-// check over every float x gives the IEEE quotient for both constants
-// whenever |x| >= 2^-100 (the largest x that differs is below 2^-102), and
-// for zero, infinite and NaN x; only smaller x can differ, and the ROI never
-// divides one (its dividends are 0 or sums of int16 trace values times an
-// inverse sigma of at least 1/256, so their magnitude is 0 or above 2^-33).
+// Moves each state's probability to its source in a grouped step's word:
+// np[to] is the sum over the states with that source, in state order.  The
+// word's structure names the few states that can reach a source, so a third
+// of the selections of a general scatter are needed; a state that does not
+// reach it adds +0.
+__device__ __forceinline__ void GroupedBackStep(uint32_t w, const float (&p)[kStates], float (&np)[kStates])
+{
+    auto bit = [&](int i) { return ((w >> i) & 1u) != 0u; };
+    constexpr int nine[5] = {0, 5, 6, 7, 8};
+    float z[5], a[5], b[5];       // to state 0, group A, group B
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+    {
+        const int s = nine[i];
+        const bool lastB = !bit(2 * s + 1), viaA = !bit(2 * s);
+        b[i] = lastB ? p[s] : 0.0f;
+        const float rest = lastB ? 0.0f : p[s];
+        a[i] = viaA ? rest : 0.0f;
+        z[i] = viaA ? 0.0f : rest;
+    }
+    np[0] = add_rn(add_rn(add_rn(add_rn(z[0], z[1]), z[2]), z[3]), z[4]);
+    const uint32_t posA = (0x2367u >> ((w >> 28) & 14u)) & 3u, posB = (0x2367u >> ((w >> 25) & 14u)) & 3u;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+    {
+        const bool fFull = bit(2 * (1 + u) + 1), fDown = bit(2 * (9 + u) + 1);     // first source
+        np[1 + u] = add_rn(fFull ? p[1 + u] : 0.0f, fDown ? p[9 + u] : 0.0f);
+        const bool inA = posA == (uint32_t)u, inB = posB == (uint32_t)u;
+        float t = add_rn(inA ? a[0] : 0.0f, fFull ? 0.0f : p[1 + u]);
+        float v = inB ? b[0] : 0.0f;
+#pragma unroll
+        for (int i = 1; i < 5; ++i)
+        {
+            t = inA ? add_rn(t, a[i]) : t;
+            v = inB ? add_rn(v, b[i]) : v;
+        }
+        np[5 + u] = add_rn(t, fDown ? 0.0f : p[9 + u]);
+        np[9 + u] = v;
+    }
+}
+
+// x / c, correctly rounded, for the ROI's constants c = sqrt(2) and sqrt(3)
+// and finite x: q = x * RN(1/c) corrected once with the exact remainder x - q c
+// (Markstein's correction).  An exhaustive check over every float x gives the
+// IEEE quotient for both constants whenever |x| >= 2^-100 (the largest x that
+// differs is below 2^-102), and zero for zero; only smaller x can differ, and
+// the ROI never divides one (its dividends are 0 or sums of int16 trace values
+// times an inverse sigma of at least 1/256, so their magnitude is 0 or above
+// 2^-33).  A zero's sign may change, which no threshold sees.
 __device__ __forceinline__ float DivByConst(float x, float c, float rcp)
 {
     const float q = mul_rn(x, rcp);
-    const float r = fma_rn(-q, c, x);
-    const float q2 = fma_rn(r, rcp, q);
-    return (isfinite(q) && q != 0.0f) ? q2 : q;
+    return fma_rn(fma_rn(-q, c, x), rcp, q);
+}
+
+// The ROI's statistic with the reference's maxima and divisions, for values
+// that may be infinite or NaN.
+__device__ __noinline__ float RoiValueGeneral(float p1, float s2, float s3, float s4, float sqrt2, float sqrt3)
+{
+    float mval = fmax_sse(p1, s2 / sqrt2);
+    mval = fmax_sse(mval, s3 / sqrt3);
+    return fmax_sse(mval, s4 / 2.0f);
 }
 
 constexpr int kBatch = 8;                              // frames loaded ahead
-
-// L1 prefetch of one address, no register result: used where the next loads
-// are needed sooner than one loop iteration can hide (the ROI pass spends ~30
-// instructions a frame) and for the traceback words read back in batches.
-__device__ __forceinline__ void PrefetchL1(const void* p) { asm volatile("prefetch.global.L1 [%0];" :: "l"(p)); }
-
 
 // Blocks per SM the labeler variants are compiled for (96 registers a thread).
 constexpr int LabelerMinBlocks(int threads) { return threads == 64 ? 10 : threads == 128 ? 5 : 2; }
@@ -400,72 +534,118 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
     if (!ZmwOf(map, A.lanes, l, z)) return;
     const int g = l * kLane + z;
     const int F = map.On() ? map.Pool(l).F : A.F;
-    const int nRoi = F + kLookback + kStitch;
     const int16_t* chunk = A.trace + map.Block(l, F) + z;
     int16_t* pl = A.prevLat + (size_t)l * kLatent * kLane + z;
     const hw_lane_model& oldM = A.latModel[l];
     const hw_lane_model& newM = A.models[l];
 
     // ---- ROI (ComputeRoi, FrameLabelerHost.cpp:267-309; RoiHost.h:110-249)
-    // 2-bit ROI codes, 16 per word, in dynamic shared memory [word][thread]
-    // (kept out of local memory, whose L1 share depends on other kernels'
-    // shared-memory carve-out).
+    // One bit a frame, 32 frames a word with the earliest in bit 31, in
+    // dynamic shared memory [word][thread] (kept out of local memory, whose
+    // L1 share depends on other kernels' shared-memory carve-out).  Bit v is
+    // frame v - 2 of the ROI block (v - 2 < F + kLookback + kStitch): with two
+    // leading bits that pass the previous chunk's last ROI value on, the 22
+    // latent frames and the chunk's batches of 8 end on whole bytes.
     extern __shared__ uint32_t roiSh[];
     auto roiw = [&](int w) -> uint32_t& { return roiSh[w * blockDim.x + threadIdx.x]; };
+    const int nWords = (F + kLatent + 31) / 32;
     {
         const float inv1 = 1.0f / sqrtf(h2f(oldM.baseline.vars[z]));
         const float inv2 = 1.0f / sqrtf(h2f(newM.baseline.vars[z]));
         float p0 = mul_rn((float)A.latTrc[g], inv1);
         float p1 = mul_rn((float)pl[0], inv1);
         float p2 = mul_rn((float)pl[kLane], inv1);
-        uint32_t prevRoi = (uint16_t)A.latRoi[g];
-        uint32_t word = 0;
-        int ri = 0;
+        uint32_t prevRoi = (uint16_t)A.latRoi[g] & 1u;
+        // a baseline variance of 0, infinity or NaN (or a NaN threshold):
+        // comparisons instead of signs, with the reference's maxima
+        const bool plain = isfinite(inv1) & isfinite(inv2) & !isnan(k.roiUpper) & !isnan(k.roiLower);
+        // complements of the bits, most recent frame in bit 0
+        uint32_t nu = prevRoi ? 1u : 3u, nl = 0u;
         auto process = [&](float sn) {
-            float mval = p1;
-            mval = fmax_sse(mval, DivByConst(p0 + p1, k.sqrt2, k.rcpSqrt2));
-            mval = fmax_sse(mval, DivByConst(add_rn(p0 + p1, p2), k.sqrt3, k.rcpSqrt3));
-            mval = fmax_sse(mval, add_rn(add_rn(p0 + p1, p2), sn) / 2.0f);
-            const float thresh = (prevRoi & 1u) ? k.roiLower : k.roiUpper;
-            const uint32_t v = ((mval >= thresh) ? 1u : 0u) | ((mval >= k.roiLower) ? 2u : 0u);
-            word |= v << (2 * (ri & 15));
-            if ((ri & 15) == 15) { roiw(ri >> 4) = word; word = 0; }
-            ++ri;
-            prevRoi = v;
+            const float s2 = p0 + p1, s3 = add_rn(s2, p2), s4 = add_rn(s3, sn);
+            if (plain)
+            {
+                const float mval = fmaxf(max3(p1, DivByConst(s2, k.sqrt2, k.rcpSqrt2),
+                                              DivByConst(s3, k.sqrt3, k.rcpSqrt3)), mul_rn(s4, 0.5f));
+                nu = PushTop<1>(nu, mval - k.roiUpper);
+                nl = PushTop<1>(nl, mval - k.roiLower);
+            }
+            else
+            {
+                const float mval = RoiValueGeneral(p1, s2, s3, s4, k.sqrt2, k.sqrt3);
+                nu = (nu << 1) | ((mval >= k.roiUpper) ? 0u : 1u);
+                nl = (nl << 1) | ((mval >= k.roiLower) ? 0u : 1u);
+            }
             p0 = p1; p1 = p2; p2 = sn;
         };
+        // Forward recursion over a word of upper (u) and lower (l) threshold
+        // bits: f = u | (l & previous f), by doubling steps; the carry is the
+        // previous word's last bit.  With the upper threshold below the lower
+        // one (previous f ? l : u), frame by frame.
+        const bool nested = k.roiUpper >= k.roiLower;
+        auto forward = [&](uint32_t u, uint32_t lw, uint32_t carry) -> uint32_t {
+            if (nested)
+            {
+                uint32_t f = u | ((carry << 31) & lw), c = lw;
+#pragma unroll
+                for (int d = 1; d < 32; d *= 2)
+                {
+                    f |= c & (f >> d);
+                    c &= c >> d;
+                }
+                return f;
+            }
+            uint32_t f = 0u;
+            for (int j = 31; j >= 0; --j)
+            {
+                carry = ((carry ? lw : u) >> j) & 1u;
+                f |= carry << j;
+            }
+            return f;
+        };
+        // forward words in roiw[0, nWords), lower-threshold words after them
+        auto flush = [&](int w, uint32_t u, uint32_t lw) {
+            const uint32_t f = forward(u, lw, prevRoi);
+            prevRoi = f & 1u;
+            roiw(w) = f;
+            roiw(nWords + w) = lw;
+        };
         for (int i = hwp::kRoiLookForward; i < kLatent; ++i) process(mul_rn((float)pl[(size_t)i * kLane], inv1));
+        int16_t x[kBatch];
+#pragma unroll
+        for (int j = 0; j < kBatch; ++j) x[j] = __ldg(chunk + (size_t)j * kLane);
+        for (int f0 = 0; f0 < F; f0 += kBatch)
         {
-            int16_t y0 = __ldg(chunk), y1 = __ldg(chunk + kLane);
-#pragma unroll 2
-            for (int i = 0; i < F; ++i)
-            {
-                if (i + 8 < F) PrefetchL1(chunk + (size_t)(i + 8) * kLane);
-                const int16_t y = y0;
-                y0 = y1;
-                if (i + 2 < F) y1 = __ldg(chunk + (size_t)(i + 2) * kLane);
-                process(mul_rn((float)y, inv2));
-            }
+            int16_t xn[kBatch];
+            const int fn = f0 + kBatch < F ? f0 + kBatch : f0;
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) xn[j] = __ldg(chunk + (size_t)(fn + j) * kLane);
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) process(mul_rn((float)x[j], inv2));
+#pragma unroll
+            for (int j = 0; j < kBatch; ++j) x[j] = xn[j];
+            const int v = f0 + kLatent + kBatch;
+            if ((v & 31) == 0) flush((v >> 5) - 1, ~nu, ~nl);
         }
-        if (ri & 15) roiw(ri >> 4) = word;
-        // Backward recursion: 2-bit codes become 0/1 (in place, bit 0 of each code).
-        uint32_t pr = 0;
-        for (int wi = (nRoi - 1) >> 4; wi >= 0; --wi)
+        const int rest = (F + kLatent) & 31;
+        if (rest) flush(nWords - 1, ~nu << (32 - rest), ~nl << (32 - rest));
+        // Backward recursion: b = f | (l & following b).
+        uint32_t next = 0u;
+        for (int w = nWords - 1; w >= 0; --w)
         {
-            uint32_t wv = roiw(wi);
-            uint32_t outw = 0;
-            const int hi = (wi == ((nRoi - 1) >> 4)) ? ((nRoi - 1) & 15) : 15;
-            for (int j = hi; j >= 0; --j)
+            uint32_t b = roiw(w), c = roiw(nWords + w);
+            b |= c & next;
+#pragma unroll
+            for (int d = 1; d < 32; d *= 2)
             {
-                const uint32_t code = (wv >> (2 * j)) & 3u;
-                const uint32_t b = (code & 1u) | (((code & 2u) != 0u) & (pr != 0u));
-                pr = b;
-                outw |= b << (2 * j);
+                b |= c & (b << d);
+                c &= c << d;
             }
-            roiw(wi) = outw;
+            next = b >> 31;
+            roiw(w) = b;
         }
     }
-    auto roiBit = [&](int f) -> bool { return (roiw(f >> 4) >> (2 * (f & 15))) & 1u; };
+    auto roiBit = [&](int f) -> bool { return (roiw((f + 2) >> 5) >> (31 - ((f + 2) & 31))) & 1u; };
 
     // ---- Viterbi (LabelBlock, FrameLabelerHost.cpp:314-448)
     StateLL ll;
@@ -480,52 +660,52 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
         return A.gap[(((size_t)l * (F + kLookback) + lf) * kStates + r) * kLane + z];
     };
     ZScorer sc;
-    auto step = [&](int lf, float x, bool isRoi) {
-        if constexpr (Margin)
-        {
-            float g[kStates];
-            tb[(size_t)lf * kLane] = ViterbiStep<true>(k, sc, x, isRoi, ll, g);
-#pragma unroll
-            for (int r = 0; r < kStates; ++r) gapAt(lf, r) = g[r];
-        }
+    // The latent frames (old model), the chunk's frames up to the anchor and
+    // the 16 look-ahead frames after it (labels kLatent .. F + 15) share one
+    // copy of the step, which is several hundred instructions.  The trace is
+    // loaded two frames ahead of use.  The log-likelihoods at the anchor wait
+    // in the ROI words' second half, which the backward recursion has used up.
+    auto anchorLL = [&](int i) -> float& { return reinterpret_cast<float&>(roiw(nWords + i)); };
+    const int nSteps = F + kLookback;
+#pragma unroll 1
+    for (int lf = 0; lf < nSteps;)
+    {
+        const int16_t* src = lf < kLatent ? pl : chunk - (size_t)kLatent * kLane;
+        const int end = lf < kLatent ? kLatent : lf < F ? F : nSteps;
+        if (lf < F) sc.Setup(k, lf < kLatent ? oldM : newM, z);
         else
         {
-            tb[(size_t)lf * kLane] = ViterbiStep<false, Grouped>(k, sc, x, isRoi, ll);
-        }
-    };
-    sc.Setup(k, oldM, z);
-    uint32_t roiWord = roiw(0);
-    for (int f = 0; f < kLatent; ++f)
-    {
-        if ((f & 15) == 0) roiWord = roiw(f >> 4);
-        const bool isRoi = (roiWord >> (2 * (f & 15))) & 1u;
-        step(f, (float)pl[(size_t)f * kLane], isRoi);
-    }
-    sc.Setup(k, newM, z);
-    const int anchor = F - kLatent;
-    float anchorLL[kStates];
-    // Chunk frames 0 .. anchor + 15 (labels kLatent .. F + 15).  The loop
-    // stays rolled (one Viterbi step is several hundred instructions; copies
-    // of it overflow the instruction cache) and the trace is loaded two
-    // frames ahead of use.
-    const int nFrames = anchor + kLookback;
-    int16_t x0 = __ldg(chunk), x1 = __ldg(chunk + kLane);
-#pragma unroll 1
-    for (int f = 0; f < nFrames; ++f)
-    {
-        const int16_t x = x0;
-        x0 = x1;
-        if (f + 2 < nFrames) x1 = __ldg(chunk + (size_t)(f + 2) * kLane);
-        if (f == anchor)
-        {
 #pragma unroll
-            for (int i = 0; i < kStates; ++i) anchorLL[i] = ll.Get(i);
+            for (int i = 0; i < kStates; ++i) anchorLL(i) = ll.Get(i);
         }
-        const int lf = f + kLatent;
-        if ((lf & 15) == 0) roiWord = roiw(lf >> 4);
-        const bool isRoi = (roiWord >> (2 * (lf & 15))) & 1u;
-        step(lf, (float)x, isRoi);
+        const bool bad = !sc.ordinary;
+        uint32_t roiWord = ~roiw((lf + 2) >> 5) << ((lf + 2) & 31);
+        int16_t x0 = __ldg(src + (size_t)lf * kLane);
+        int16_t x1 = __ldg(src + (size_t)(lf + 1 < end ? lf + 1 : lf) * kLane);
+#pragma unroll 1
+        for (; lf < end; ++lf)
+        {
+            const float x = (float)x0;
+            x0 = x1;
+            if (lf + 2 < end) x1 = __ldg(src + (size_t)(lf + 2) * kLane);
+            if (((lf + 2) & 31) == 0) roiWord = ~roiw((lf + 2) >> 5);
+            // 0 on an ROI frame, -inf on another
+            const float npen = __int_as_float(((int)roiWord >> 31) & (int)0xff800000);
+            roiWord <<= 1;
+            uint32_t w;
+            if constexpr (Margin)
+            {
+                float gp[kStates];
+                w = ViterbiStep<true>(k, sc, x, npen, ll, gp);
+#pragma unroll
+                for (int r = 0; r < kStates; ++r) gapAt(lf, r) = gp[r];
+            }
+            else if constexpr (Grouped) w = GroupedStep(k, sc, x, npen, bad, ll);
+            else w = ViterbiStep<false>(k, sc, x, npen, ll);
+            tb[(size_t)lf * kLane] = w;
+        }
     }
+    const int anchor = F - kLatent;
 
     // Normalize (FrameLabelerHost.cpp:186-205) and back-propagation.
     float prob[kStates];
@@ -545,14 +725,18 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
     {
         const uint32_t w = tb[(size_t)i * kLane];
         float np[kStates];
-#pragma unroll
-        for (int s = 0; s < kStates; ++s) np[s] = 0.0f;
-#pragma unroll
-        for (int from = 0; from < kStates; ++from)
+        if (Grouped && !(w & kGenericWord)) GroupedBackStep(w, prob, np);
+        else
         {
-            const int to = TraceSource(w, from);
 #pragma unroll
-            for (int s = 0; s < kStates; ++s) np[s] = (s == to) ? add_rn(np[s], prob[from]) : np[s];
+            for (int s = 0; s < kStates; ++s) np[s] = 0.0f;
+#pragma unroll
+            for (int from = 0; from < kStates; ++from)
+            {
+                const int to = GenericSource(Grouped ? w >> kGenericShift : w, from);
+#pragma unroll
+                for (int s = 0; s < kStates; ++s) np[s] = (s == to) ? add_rn(np[s], prob[from]) : np[s];
+            }
         }
 #pragma unroll
         for (int s = 0; s < kStates; ++s) prob[s] = np[s];
@@ -566,9 +750,7 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
         maxP = c ? maxP : prob[i];
         anchorState = c ? anchorState : i;
     }
-    float ret = anchorLL[0];
-#pragma unroll
-    for (int i = 1; i < kStates; ++i) ret = (anchorState == i) ? anchorLL[i] : ret;
+    const float ret = anchorLL(anchorState);
 
     int ts = anchorState;
     if constexpr (Fuse)
@@ -591,7 +773,7 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
             for (int j = kBatch - 1; j >= 0; --j)
             {
                 word |= (uint32_t)ts << (4 * j);
-                ts = TraceSource(w[j], ts);
+                ts = TraceSource<Grouped>(w[j], ts);
             }
             roiw(f0 / kBatch) = word;
         }
@@ -637,7 +819,7 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
             out[(size_t)f * kLane] = (int16_t)ts;
             if (f < F - 1) mg[(size_t)f * kLane] = gapAt(f + 1, next);
             next = ts;
-            ts = TraceSource(tb[(size_t)f * kLane], ts);
+            ts = TraceSource<Grouped>(tb[(size_t)f * kLane], ts);
         }
         A.latRoi[g] = (int16_t)roiBit(F - 1);
     }
@@ -660,7 +842,7 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
             for (int j = kBatch - 1; j >= 0; --j)
             {
                 out[(size_t)(f0 + j) * kLane] = (int16_t)ts;
-                ts = TraceSource(w[j], ts);
+                ts = TraceSource<Grouped>(w[j], ts);
             }
         }
         A.latRoi[g] = (int16_t)roiBit(F - 1);
@@ -689,14 +871,20 @@ __global__ void LabelerModelCopyKernel(hw_lane_model* dst, const hw_lane_model* 
     reinterpret_cast<uint32_t*>(dst)[w] = reinterpret_cast<const uint32_t*>(src)[w];
 }
 
+// Shared-memory words a thread: the ROI words twice (the second half also
+// holds the anchor's log-likelihoods), packed labels after them (fused).
+constexpr int LabelerWords(int F, bool fuse)
+{
+    const int n = (F + kLatent + 31) / 32;
+    const int words = n + (n > kStates ? n : kStates);
+    return fuse && F / kBatch > words ? F / kBatch : words;
+}
+
 template <bool Mapped, bool Fuse, int Threads, bool Margin = false, bool Grouped = false>
 cudaError_t LaunchLabelerT(const LabelerArgs& a, const KParams& k, const PulseArgs& p, int lanes, cudaStream_t s)
 {
     const int blocks = (lanes * kLane + Threads - 1) / Threads;
-    // ROI words during the forward pass, packed labels after it (fused)
-    const int roiWords = (a.F + kLookback + kStitch + 15) / 16;
-    const int words = Fuse ? (roiWords > a.F / kBatch ? roiWords : a.F / kBatch) : roiWords;
-    const size_t smem = (size_t)words * Threads * sizeof(uint32_t);
+    const size_t smem = (size_t)LabelerWords(a.F, Fuse) * Threads * sizeof(uint32_t);
     static bool attrSet[64] = {};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -705,9 +893,7 @@ cudaError_t LaunchLabelerT(const LabelerArgs& a, const KParams& k, const PulseAr
     {
         e = cudaFuncSetAttribute(LabelerKernel<Mapped, Fuse, Threads, Margin, Grouped>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)(((1024 + kLookback + kStitch + 15) / 16 > 1024 / kBatch
-                                            ? (1024 + kLookback + kStitch + 15) / 16 : 1024 / kBatch) *
-                                       Threads * sizeof(uint32_t)));
+                                 (int)(LabelerWords(1024, Fuse) * Threads * sizeof(uint32_t)));
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 64) attrSet[dev] = true;
     }

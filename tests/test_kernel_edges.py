@@ -80,6 +80,57 @@ def test_estimate_paths(kind):
     _both(cfg, lanes, 512, lambda b: b.estimate(hist, stats, (0, 4096), (0, 512), prior))
 
 
+def _models(lanes, seed=0):
+    import oracle
+    cfg = workloads.small_config()
+    cfg.model_estimation_mode = abi.FIXED_ESTIMATIONS
+    m = oracle.static_model(cfg, lanes)
+    rng = np.random.default_rng(seed)
+    for a, amp in enumerate(workloads.AMPLITUDES_DN):
+        g = rng.lognormal(0.0, 0.2, (lanes, abi.LANE)).astype(np.float32)
+        m["analogs"]["means"][:, a] = abi.f32_to_f16(amp * g)
+        m["analogs"]["vars"][:, a] = abi.f32_to_f16(64.0 + 0.5 * amp * g + 0.01 * (amp * g) ** 2)
+    m["baseline"]["means"] = abi.f32_to_f16(np.zeros((lanes, abi.LANE)))
+    m["baseline"]["vars"] = abi.f32_to_f16(np.full((lanes, abi.LANE), 64.0))
+    return m
+
+
+@pytest.mark.parametrize("kind", ["plain", "equal_analogs", "below_baseline", "zero_var", "inf_var", "reversed_roi",
+                                  "open_roi"])
+@pytest.mark.parametrize("F", [48, 208, 1024])
+def test_label_paths(kind, F):
+    lanes = 3
+    cfg = workloads.small_config()
+    m = _models(lanes)
+    odd = slice(1, None, 3)
+    if kind == "equal_analogs":
+        for f in ("means", "vars"):
+            m["analogs"][f][:, 1:, odd] = m["analogs"][f][:, :1, odd]
+    elif kind == "below_baseline":
+        m["analogs"]["means"][:, 2, odd] = abi.f32_to_f16(np.float32(-30.0))
+    elif kind == "zero_var":
+        m["baseline"]["vars"][:, odd] = 0
+        m["analogs"]["vars"][:, 0, odd] = 0
+    elif kind == "inf_var":
+        m["baseline"]["vars"][:, odd] = 0x7c00
+        m["analogs"]["vars"][:, 3, odd] = 0x7c00
+    elif kind == "reversed_roi":
+        cfg.roi_upper_threshold, cfg.roi_lower_threshold = 2.0, 7.0
+    elif kind == "open_roi":
+        cfg.roi_upper_threshold = cfg.roi_lower_threshold = -1e9
+    tr = synth.traces(lanes, 4 * F, seed=F, gain_sigma=0.2, empty_fraction=0.1, baseline=0.0)
+    if kind == "plain":
+        tr[0, ::97] = 32767
+        tr[1, ::89] = -32768
+
+    def call(b):
+        out = []
+        for c in range(4):
+            out += b.label(np.ascontiguousarray(tr[:, c * F:(c + 1) * F]), m)
+        return out
+    _both(cfg, lanes, F, call)
+
+
 @pytest.mark.parametrize("F", [48, 512])
 @pytest.mark.parametrize("pedestal,sensitivity,extreme", [(0, 1.0, False), (13, 1.9, False), (-32768, 0.01, True),
                                                           (32767, 62.0, True), (5, 100.0, True), (0, 3.0e7, False)])
