@@ -161,9 +161,6 @@ __device__ __forceinline__ int HistBin(float v)
     return (v >= (float)kBins && v < 2147483648.0f) ? kBins : -1;
 }
 
-// int16 -> float, exactly: 1.5 x 2^23 + x has the bit pattern 0x4B400000 + x.
-__device__ __forceinline__ float I16ToFloat(int16_t x) { return __int_as_float(0x4B400000 + (int)x) - 12582912.0f; }
-
 // AddBlock (TraceHistogramAccumHost.cpp:140-169): edge scrubbing with the fp16
 // baseline mode, then UHistogramSimd::AddDatum.  Counts of the lane are held
 // in shared memory for the chunk (one u16 per bin and ZMW; each thread only
@@ -261,6 +258,76 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
                 cnt[ll][bb][z] = (uint16_t)(cb + 1);
             }
         };
+        // One batch of frames of both halves: the bins of all its frames first
+        // (independent, so their arithmetic overlaps), then the counts.  The
+        // quotient is formed with the reciprocal of the bin size: two
+        // corrections by the exact remainder (Markstein) give the IEEE
+        // quotient when the reciprocal is correctly rounded and nothing
+        // under- or overflows, which `plainDiv` ensures (a quotient whose
+        // remainder underflows is far below 1 and keeps its sign).  A
+        // division instead is twice the instructions and a branch a frame,
+        // which kept the frames' chains from overlapping (reset, 8 chunks of
+        // 2048 lanes x 512 frames and read-out: 1490 -> 1295 us).  Chunks
+        // whose frames fill no whole batches, bin sizes out of range and a
+        // classifier without two frames of history take the division.
+        const float rcpBin = 1.0f / binSize;
+        const bool plainDiv = binSize > 9.094947017729282e-13f && binSize < 1.099511627776e12f &&
+                              fabsf(lower) < 1.099511627776e12f;          // 2^-40, 2^40
+        auto fast = [&](const int16_t (&xA)[kHistPairBatch], const int16_t (&xB)[kHistPairBatch]) {
+            float v[2][kHistPairBatch];
+            bool sel[2][kHistPairBatch];
+#pragma unroll
+            for (int j = 0; j < kHistPairBatch; ++j)
+            {
+                const bool isA = xA[j] < thr, isB = xB[j] < thr;
+                sel[0][j] = isA == b2;
+                sel[1][j] = isB == b2B;
+                b2 = b1; b1 = isA;
+                b2B = b1B; b1B = isB;
+                const float dA = I16ToFloat(j ? xA[j ? j - 1 : 0] : prev) - lower;
+                const float dB = I16ToFloat(j ? xB[j ? j - 1 : 0] : prevB) - lower;
+                v[0][j] = DivRcp(dA, binSize, rcpBin);
+                v[1][j] = DivRcp(dB, binSize, rcpBin);
+            }
+            prev = xA[kHistPairBatch - 1];
+            prevB = xB[kHistPairBatch - 1];
+            bool outlier = false;
+#pragma unroll
+            for (int j = 0; j < kHistPairBatch; ++j)
+            {
+                const bool inA = (v[0][j] >= 0.0f) & (v[0][j] < (float)kBins);
+                const bool inB = (v[1][j] >= 0.0f) & (v[1][j] < (float)kBins);
+                outlier |= (sel[0][j] & !inA) | (sel[1][j] & !inB);
+                // floor(v) from v + 2^23 rounded down (see HistBin)
+                const int fA = __float_as_int(__fadd_rd(v[0][j], 8388608.0f)) - 0x4B000000;
+                const int fB = __float_as_int(__fadd_rd(v[1][j], 8388608.0f)) - 0x4B000000;
+                const int ba = (sel[0][j] & inA) ? fA : kBins, bb = (sel[1][j] & inB) ? fB : kBins;
+                const uint16_t ca = cnt[ll][ba][z], cb = cnt[ll][bb][z];
+                const uint16_t one = ba == bb ? 2 : 1;
+                cnt[ll][ba][z] = (uint16_t)(ca + one);
+                if (ba != bb) cnt[ll][bb][z] = (uint16_t)(cb + 1);
+            }
+            if (outlier)
+            {
+#pragma unroll
+                for (int j = 0; j < kHistPairBatch; ++j)
+                {
+                    const int fA = sel[0][j] ? HistBin(v[0][j]) : 0, fB = sel[1][j] ? HistBin(v[1][j]) : 0;
+                    nLow = (uint16_t)(nLow + (fA < 0 ? 1 : 0));
+                    nHigh = (uint16_t)(nHigh + (fA >= kBins ? 1 : 0));
+                    nLowB = (uint16_t)(nLowB + (fB < 0 ? 1 : 0));
+                    nHighB = (uint16_t)(nHighB + (fB >= kBins ? 1 : 0));
+                }
+            }
+        };
+        auto batch = [&](const int16_t (&xA)[kHistPairBatch], const int16_t (&xB)[kHistPairBatch]) {
+            if (plainDiv && n == 2) fast(xA, xB);
+            else
+            {
+#pragma unroll
+                for (int j = 0; j < kHistPairBatch; ++j) pair(xA[j], xB[j]);
+            }
+        };
         int16_t aA[kHistPairBatch], aB[kHistPairBatch], bA[kHistPairBatch], bB[kHistPairBatch];
 #pragma unroll
         for (int j = 0; j < kHistPairBatch; ++j)
@@ -269,6 +336,7 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
             aB[j] = __ldg(tr + (size_t)(S + j) * kLane);
         }
         int i = 0;
+#pragma unroll 1
         for (; i + 2 * kHistPairBatch <= S; i += 2 * kHistPairBatch)
         {
 #pragma unroll
@@ -277,8 +345,7 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
                 bA[j] = __ldg(tr + (size_t)(i + kHistPairBatch + j) * kLane);
                 bB[j] = __ldg(tr + (size_t)(S + i + kHistPairBatch + j) * kLane);
             }
-#pragma unroll
-            for (int j = 0; j < kHistPairBatch; ++j) pair(aA[j], aB[j]);
+            batch(aA, aB);
             if (i + 3 * kHistPairBatch <= S)
             {
 #pragma unroll
@@ -288,8 +355,7 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
                     aB[j] = __ldg(tr + (size_t)(S + i + 2 * kHistPairBatch + j) * kLane);
                 }
             }
-#pragma unroll
-            for (int j = 0; j < kHistPairBatch; ++j) pair(bA[j], bB[j]);
+            batch(bA, bB);
         }
         // S is a multiple of 2 x kHistPairBatch: nothing is left over
         nLow = (uint16_t)(nLow + nLowB);
