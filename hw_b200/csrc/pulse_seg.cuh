@@ -11,13 +11,22 @@
 
 namespace hwk {
 
-__device__ __forceinline__ uint16_t ToFixed(float v) { return static_cast<uint16_t>(add_rn(v / .1f, 0.5f)); }
+// v is 0 or at least 2^-17 (a sum of int16 values over a width): v / .1f, with
+// 10 the correctly rounded reciprocal of .1f.
+__device__ __forceinline__ uint16_t ToFixed(float v)
+{
+    return static_cast<uint16_t>(add_rn(DivRcp(v, .1f, 10.0f), 0.5f));
+}
 
-// The open segment (LabelsSegment) and the chunk's outputs of one ZMW.
+// The open segment (LabelsSegment) and the chunk's outputs of one ZMW.  The
+// int16 signals are held as floats (their sums are float sums, and the
+// maximum of exact floats is that of the integers), so a frame converts its
+// signal once.
 struct PulseSeg
 {
     uint32_t start;
-    int16_t first, last, mx, label;
+    int label;
+    float first, last, mx;
     float total, m2;
     uint32_t n, over;
     float b0, b1, b2;       // StatAccumulator of baseline frames (offset 0)
@@ -28,12 +37,13 @@ struct PulseSeg
     uint32_t pStart;
     int pWidth;
     float pNum, pTotal, pM2;       // (total + last) + first, total, m2
-    int16_t pMx, pLabel;
+    float pMx;
+    int pLabel;
 
     __device__ __forceinline__ void Load(const PulseArgs& A, int g, float minMeanIn, hw_pulse* outIn)
     {
         start = A.segStart[g];
-        first = A.segFirst[g]; last = A.segLast[g]; mx = A.segMax[g]; label = A.segLabel[g];
+        first = (float)A.segFirst[g]; last = (float)A.segLast[g]; mx = (float)A.segMax[g]; label = A.segLabel[g];
         total = A.segTotal[g]; m2 = A.segM2[g];
         n = 0; over = 0;
         b0 = 0.0f; b1 = 0.0f; b2 = 0.0f;
@@ -57,7 +67,7 @@ struct PulseSeg
         p.width = (uint16_t)width;
         p.mean_signal = ToFixed(fmin_std(maxSignal, fmax_std(minSignal, rawMean)));
         p.mid_signal = ToFixed(width < 3 ? 0.0f : fmin_std(maxSignal, fmax_std(minSignal, rawMid)));
-        p.max_signal = ToFixed(fmin_std(maxSignal, fmax_std(minSignal, (float)pMx)));
+        p.max_signal = ToFixed(fmin_std(maxSignal, fmax_std(minSignal, pMx)));
         p.signal_m2 = pM2;
         int lbl = pLabel;
         if (lbl > 2 * kAnalogs) lbl -= 2 * kAnalogs;
@@ -80,11 +90,16 @@ struct PulseSeg
         }
     }
 
-    __device__ __forceinline__ void Frame(const KParams& k, uint32_t absF, int16_t lb, int16_t signal)
+    // One frame with its label and signal.  The segment's sums advance by
+    // selects: some ZMW of a warp starts a segment in nearly every frame, so a
+    // branch would run both sides (71 -> 56 warp instructions a frame with the
+    // single conversion, 613 lanes x 256 frames packed: 80 -> 66 us).
+    __device__ __forceinline__ void Frame(const KParams& k, uint32_t absF, int lb, float signal)
     {
-        const bool isUp = (lb > kAnalogs) & (lb <= 2 * kAnalogs);
-        const bool boundary = isUp | ((lb == 0) & (label != 0));
+        const bool isUp = (unsigned)(lb - (kAnalogs + 1)) < (unsigned)kAnalogs;
         const bool pulseM = label != 0;
+        const bool boundary = isUp | ((lb == 0) & pulseM);
+        const float t1 = add_rn(total, last);
         if (boundary & pulseM)
         {
             // The pulse's raw sums wait in the pending slot; ToPulse runs at
@@ -94,35 +109,35 @@ struct PulseSeg
             pend = true;
             pStart = start;
             pWidth = (int)(absF - start);
-            pNum = add_rn(add_rn(total, (float)last), (float)first);
+            pNum = add_rn(t1, first);
             pTotal = total;
             pM2 = m2;
             pMx = mx;
             pLabel = label;
         }
-        if (boundary)
+        const float m1 = add_rn(m2, mul_rn(last, last));
+        const float mx1 = fmaxf(mx, signal);
+        if (!(pulseM | boundary))
         {
-            start = absF; first = signal; last = 0; mx = signal; total = 0.0f; m2 = 0.0f; label = lb;
+            b0 += 1.0f;
+            b1 = add_rn(b1, signal);
+            b2 = add_rn(b2, mul_rn(signal, signal));
         }
-        else
-        {
-            total = add_rn(total, (float)last);
-            m2 = add_rn(m2, mul_rn((float)last, (float)last));
-            last = signal;
-            mx = signal > mx ? signal : mx;
-        }
-        if ((!pulseM) & (!boundary))
-        {
-            const float x = (float)signal;
-            b0 += 1.0f; b1 = add_rn(b1, x); b2 = add_rn(b2, mul_rn(x, x));
-        }
+        start = boundary ? absF : start;
+        label = boundary ? lb : label;
+        first = boundary ? signal : first;
+        mx = boundary ? signal : mx1;
+        total = boundary ? 0.0f : t1;
+        m2 = boundary ? 0.0f : m1;
+        last = boundary ? 0.0f : signal;
     }
 
     __device__ __forceinline__ void Store(const PulseArgs& A, int g, int l, int z, uint32_t* lensOut,
                                           uint32_t* ovfOut, int go) const
     {
-        A.segStart[g] = start; A.segFirst[g] = first; A.segLast[g] = last; A.segMax[g] = mx;
-        A.segTotal[g] = total; A.segM2[g] = m2; A.segLabel[g] = label;
+        A.segStart[g] = start; A.segFirst[g] = (int16_t)first; A.segLast[g] = (int16_t)last;
+        A.segMax[g] = (int16_t)mx;
+        A.segTotal[g] = total; A.segM2[g] = m2; A.segLabel[g] = (int16_t)label;
         lensOut[go] = n;
         ovfOut[go] = over;
         A.bls[l].offset[z] = 0.0f;

@@ -27,21 +27,35 @@ __global__ void __launch_bounds__(128) PulseKernel(PulseArgs A, KParams k)
     const int16_t* lab = A.labels + A.map.Block(l, F) + z;
     const int16_t* lat = A.latTrace + (size_t)l * kLatent * kLane + z;
     const int16_t* tr = A.trace + A.map.Block(l, F) + z;
+    // Labels and signals in two register batches of 8 frames that alternate,
+    // each loaded while the other is accumulated (F % 8 == 0, and the latent
+    // traces end with a batch).
     constexpr int kB = 8;
-    for (int rel0 = 0; rel0 < F; rel0 += kB)
-    {
-        // Load the next kB labels and signals ahead of use (F % 8 == 0).
-        int16_t lbB[kB], sgB[kB];
+    static_assert(kLatent % kB == 0, "a batch lies in the latent traces or in the chunk");
+    auto load = [&](int rel0, int16_t (&lb)[kB], int16_t (&sg)[kB]) {
+        const int16_t* src = rel0 < kLatent ? lat + (size_t)rel0 * kLane : tr + (size_t)(rel0 - kLatent) * kLane;
+        const int16_t* ls = lab + (size_t)rel0 * kLane;
 #pragma unroll
         for (int j = 0; j < kB; ++j)
         {
-            const int r = rel0 + j;
-            lbB[j] = __ldg(lab + (size_t)r * kLane);
-            sgB[j] = (r < kLatent) ? __ldg(lat + (size_t)r * kLane) : __ldg(tr + (size_t)(r - kLatent) * kLane);
+            lb[j] = __ldg(ls + (size_t)j * kLane);
+            sg[j] = __ldg(src + (size_t)j * kLane);
         }
+    };
+    auto accumulate = [&](int rel0, const int16_t (&lb)[kB], const int16_t (&sg)[kB]) {
 #pragma unroll
-        for (int j = 0; j < kB; ++j) seg.Frame(k, (uint32_t)(rel0 + j) + firstFrame, lbB[j], sgB[j]);
+        for (int j = 0; j < kB; ++j) seg.Frame(k, (uint32_t)(rel0 + j) + firstFrame, lb[j], I16ToFloat(sg[j]));
         seg.Flush(k);
+    };
+    int16_t lbA[kB], sgA[kB], lbB[kB], sgB[kB];
+    load(0, lbA, sgA);
+#pragma unroll 1
+    for (int rel0 = 0; rel0 < F; rel0 += 2 * kB)
+    {
+        if (rel0 + kB < F) load(rel0 + kB, lbB, sgB);
+        accumulate(rel0, lbA, sgA);
+        if (rel0 + 2 * kB < F) load(rel0 + 2 * kB, lbA, sgA);
+        if (rel0 + kB < F) accumulate(rel0 + kB, lbB, sgB);
     }
     seg.Store(A, g, l, z, ps ? ps->lens : A.lens, ps ? ps->ovf : A.ovf, go);
 }
