@@ -46,14 +46,12 @@ constexpr size_t kParams = kOffB3 + kOut;
 constexpr int kFeatThreads = 256;
 
 // Per ZMW: the inverse of the in-range count total and the two baseline
-// features (shared by the features kernel and the fused proposal).
-__device__ __forceinline__ void FeatureRow(const hw_lane_histogram& H, const hw_baseliner_stats& st, int z,
-                                           float& inv, float& fMean, float& fVar)
+// features (shared by the features kernel and the fused proposal).  `count` is
+// the integer total (below 2^24 for any histogram the accumulator fills, so
+// equal to the float sum in any order).
+__device__ __forceinline__ void RowFeatures(uint32_t count, const hw_lane_histogram& H, const hw_baseliner_stats& st,
+                                            int z, float& inv, float& fMean, float& fVar)
 {
-    // the integer total (below 2^24 for any histogram the accumulator fills,
-    // so equal to the float sum in any order)
-    uint32_t count = 0;
-    for (int b = 0; b < kBins; ++b) count += H.bin_count[b][z];
     const float total = (float)count;
     inv = total > 0.0f ? 1.0f / total : 0.0f;
     const float lb = H.low_bound[z], bs = H.bin_size[z];
@@ -64,6 +62,14 @@ __device__ __forceinline__ void FeatureRow(const hw_lane_histogram& H, const hw_
     const float fm = (mean - lb) / bs, fv = var / (bs * bs);
     fMean = isfinite(fm) ? fm : 0.0f;
     fVar = isfinite(fv) ? fv : 0.0f;
+}
+
+__device__ __forceinline__ void FeatureRow(const hw_lane_histogram& H, const hw_baseliner_stats& st, int z,
+                                           float& inv, float& fMean, float& fVar)
+{
+    uint32_t count = 0;
+    for (int b = 0; b < kBins; ++b) count += H.bin_count[b][z];
+    RowFeatures(count, H, st, z, inv, fMean, fVar);
 }
 
 __device__ __forceinline__ float FeatureValue(const hw_lane_histogram& H, int z, int b, float inv, float fMean,
@@ -162,10 +168,14 @@ template <typename T> __device__ __forceinline__ __nv_bfloat16 ToBf16(T v);
 template <> __device__ __forceinline__ __nv_bfloat16 ToBf16<float>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 ToBf16<__nv_bfloat16>(__nv_bfloat16 v) { return v; }
 
+// 0.5 x (1 + tanh(u)) = x / (1 + exp(-2 u)), u = k0 (x + k1 x^3): no
+// cancellation where the tanh is near -1, and a third of the instructions.
 __device__ __forceinline__ float GeluTanh(float x)
 {
-    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-    return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
+    const float k0 = 0.7978845608028654f, k1 = 0.044715f, c = -2.0f * 1.4426950408889634f * k0;
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * fmaf(x * x, c * k1, c)));
+    return __fdividef(x, 1.0f + e);
 }
 
 __device__ __forceinline__ float GeluTanhGrad(float x)
@@ -274,21 +284,34 @@ __global__ void __launch_bounds__(128) GemmKernel(const TA* __restrict__ A, long
 // the next 8-row group K * 16 bytes on); one thread issues
 // tcgen05.mma.cta_group::1.kind::f16 (M = 128, K = 16 a step) into a
 // 256-column FP32 accumulator in tensor memory and commits to an mbarrier;
-// the four warps read their 32 rows back (tcgen05.ld 32x32b), add the bias,
-// apply GELU and write the BF16 activations over the input tile as the next
-// layer's A operand.  Layer 1 runs as two N = 128 halves so that a weight
-// half (76 KB) and the input tile (76 KB) fit beside each other; layer 2
-// takes all of W2 (128 KB).  Rounding points are those of the mma.sync
-// path (BF16 inputs and activations, FP32 accumulation and epilogue); only
-// the order of the FP32 accumulation differs.  Every wait on the mbarrier
-// is bounded: past about a second the CTA writes NaN rows (a proposal the
-// DME's fallback test rejects), sets *err and returns.
+// all 16 warps read their rows back (tcgen05.ld 32x32b), add the bias, apply
+// GELU and write the BF16 activations over the input tile as the next layer's
+// A operand.  The weights lie in global memory in the operand's own layout, so
+// a block of them is one bulk copy (cp.async.bulk, completing on an mbarrier)
+// that runs beside the other work: W1 (two copies, 128 and 112 of its 256 rows)
+// beside the input staging, its last 16 rows, which do not fit beside the input
+// tile, beside the second product; W2 and W3 beside the epilogues.  Rounding
+// points are those of the mma.sync path (BF16 inputs and activations, FP32
+// accumulation and epilogue); only the order of the FP32 accumulation differs.
+// Every wait on an mbarrier is bounded: past about a second the CTA writes NaN
+// rows (a proposal the DME's fallback test rejects), sets *err and returns.
+//
+// Bound by the scalar work of a tile (features, standardisation, GELU): one CTA
+// a SM by shared memory, the products a few us of the tile.  262,144 rows from
+// the histograms: 973 us with weights staged by the threads, a division and a
+// square root for every input and tanhf; 420 us as written (190 TFLOP/s).
 constexpr int kTcRows = 128;
 constexpr int kTcThreads = 512;        // 16 warps: warp w reads TMEM lanes 32 (w % 4) .. + 31
 constexpr uint32_t kTcCols = 256;                                      // TMEM columns
 constexpr int kTcA = kTcRows * kFeat * 2;                             // 77,824 B: input tile, then activations
-constexpr int kTcW = kHidden * kHidden * 2;                           // 131,072 B: the largest weight block
+constexpr int kTcW1a = 128 * kFeat * 2, kTcW1b = 112 * kFeat * 2, kTcW1c = 16 * kFeat * 2;
+constexpr int kTcW2 = kHidden * kHidden * 2, kTcW3 = kOut * kHidden * 2;
+constexpr int kTcW = kTcW1a + kTcW1b;                                 // 145,920 B: the weights in use
 constexpr int kTcSmem = kTcA + kTcW;
+// weight blocks in operand layout: W1 (its three parts in turn), W2, W3
+constexpr size_t kPackW2 = (size_t)kHidden * kFeat, kPackW3 = kPackW2 + (size_t)kHidden * kHidden;
+constexpr size_t kPackAll = kPackW3 + (size_t)kOut * kHidden;
+static_assert(kTcW2 <= kTcW && kTcW3 <= kTcW && kTcW1c <= kTcW1a, "weight blocks fit their region");
 
 __device__ __forceinline__ uint32_t SmemU32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -333,12 +356,18 @@ __device__ __forceinline__ bool WaitMmas(uint32_t bar, uint32_t parity)
 }
 
 // Issued by one thread: D[tmem] (+)= A (128 x K) . B (N x K)^T over K / 16 steps.
-__device__ __forceinline__ void MmaChain(uint32_t d, uint32_t a, uint32_t b, int k, int n, uint32_t bar)
+__device__ __forceinline__ void MmaIssue(uint32_t d, uint32_t a, uint32_t b, int k, int n)
 {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t sbo = (uint32_t)k * 16u, idesc = UmmaIdesc(n);
     for (int s = 0; s < k / 16; ++s)
         UmmaBf16(d, UmmaDesc(a + s * 256u, 128u, sbo), UmmaDesc(b + s * 256u, 128u, sbo), idesc, s > 0);
+}
+
+// The same, and `bar` completes when these and all earlier products have.
+__device__ __forceinline__ void MmaChain(uint32_t d, uint32_t a, uint32_t b, int k, int n, uint32_t bar)
+{
+    MmaIssue(d, a, b, k, n);
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar)
                  : "memory");
 }
@@ -349,18 +378,36 @@ __device__ __forceinline__ uint32_t CoreOffset(int r, int c, int k)
     return (uint32_t)((r >> 3) * k * 16 + c * 128 + (r & 7) * 16);
 }
 
-// rows x k BF16 weights (row stride k) into the canonical layout, 32 bytes a task.
-__device__ __forceinline__ void StageWeights(const __nv_bfloat16* __restrict__ w, int rows, int k, uint8_t* dst)
+// The BF16 weight blocks from their row-major copy into operand layout: blocks
+// of 8 rows lie K * 16 bytes apart whatever the block's height, so any run of
+// whole 8-row groups is one contiguous piece.
+__global__ void PackWeightsKernel(const __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wp)
 {
-    const int pairs = k / 16;
-    for (int t = threadIdx.x; t < rows * pairs; t += kTcThreads)
-    {
-        const int r8 = t & 7, rest = t >> 3, c2 = rest % pairs, g = rest / pairs, r = g * 8 + r8;
-        const uint4* src = reinterpret_cast<const uint4*>(w + (size_t)r * k + c2 * 16);
-        const uint4 lo = __ldg(src), hi = __ldg(src + 1);
-        *reinterpret_cast<uint4*>(dst + CoreOffset(r, 2 * c2, k)) = lo;
-        *reinterpret_cast<uint4*>(dst + CoreOffset(r, 2 * c2 + 1, k)) = hi;
-    }
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    auto put = [&](int i, size_t src, size_t dst, int k) {
+        const int r = i / k, c = i % k;
+        wp[dst + (CoreOffset(r, c / 8, k) / 2 + (c & 7))] = wb[src + i];
+    };
+    if (e < (int)kPackW2) put(e, kOffW1, 0, kFeat);
+    else if (e < (int)kPackW3) put(e - (int)kPackW2, kOffW2, kPackW2, kHidden);
+    else if (e < (int)kPackAll) put(e - (int)kPackW3, kOffW3, kPackW3, kHidden);
+}
+
+// One thread: `bytes` of weights into shared memory, completing on `bar`.
+__device__ __forceinline__ void LoadWeights(uint32_t dst, const __nv_bfloat16* src, uint32_t bytes, uint32_t bar)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+
+// One thread: bounded wait for phase `parity` of `bar`.
+__device__ __forceinline__ bool WaitLoad(uint32_t bar, uint32_t parity)
+{
+    const long long t0 = clock64();
+    while (!MbarTryWait(bar, parity))
+        if (clock64() - t0 > 4000000000ll) return MbarTryWait(bar, parity);
+    return true;
 }
 
 // The standardised input tile (rows past n are 0), as InputKernel rounds it.
@@ -401,51 +448,129 @@ __device__ __forceinline__ void StageInput(const float* __restrict__ feat, long 
     }
 }
 
+// Per input column: mean, scale, RN(1 / scale) and the standardised value of an
+// empty bin; and the packed values of each 8-column chunk of empty bins.
+struct InputTable
+{
+    float4 col[kFeat];
+    uint4 empty[kFeat / 8];
+};
+
+// (f - mean) / scale of a histogram feature (f in [0, 1]): the IEEE quotient by
+// the reciprocal (DivRcp) where nothing can under- or overflow, marked by a
+// reciprocal that is not 0.
+__device__ __forceinline__ float Standardise(float f, float4 c)
+{
+    const float d = f - c.x;
+    return c.z != 0.0f ? DivRcp(d, c.y, c.z) : d / c.y;
+}
+
 // The same tile computed from the lanes' histograms and baseliner statistics
-// (FeatureRow / FeatureValue, as FeaturesKernel): rows are ZMWs of the lanes
-// row0 / 64 and the next.
+// (as FeatureRow / FeatureValue): rows are ZMWs of the lanes row0 / 64 and the
+// next.  A warp takes 32 ZMWs, so a bin's counts are one 64-byte row; threads
+// 128 apart share a ZMW and split its bins.  Bins empty for the whole warp
+// (most of the range) take their chunk's constant.  Sums use dst as scratch.
 __device__ __forceinline__ void StageInputFromHist(const hw_lane_histogram* __restrict__ hist,
                                                    const hw_baseliner_stats* __restrict__ st, long row0, long n,
                                                    const float* __restrict__ mean, const float* __restrict__ scale,
-                                                   uint8_t* dst, float* rowInv, float* rowMean, float* rowVar)
+                                                   uint8_t* dst, InputTable& tab, float* rowInv, float* rowMean,
+                                                   float* rowVar)
 {
-    if (threadIdx.x < kTcRows)
+    constexpr int kParts = kTcThreads / kTcRows, kBinChunks = kBins / 8;      // 37 whole chunks, bins 0..295
+    const int r = threadIdx.x & (kTcRows - 1), part = threadIdx.x / kTcRows;
+    const long row = row0 + r;
+    const bool valid = row < n;
+    const hw_lane_histogram& H = hist[valid ? row / kLane : 0];
+    const int z = (int)(row % kLane);
+    for (int c = threadIdx.x; c < kFeat; c += kTcThreads)
     {
-        const long row = row0 + threadIdx.x;
-        if (row < n)
-            FeatureRow(hist[row / kLane], st[row / kLane], (int)(row % kLane), rowInv[threadIdx.x],
-                       rowMean[threadIdx.x], rowVar[threadIdx.x]);
+        const float m = mean[c], s = scale[c];
+        const bool plain = (m == 0.0f || fabsf(m) > 9.094947017729282e-13f) && fabsf(m) < 1.099511627776e12f &&
+                           s > 9.094947017729282e-13f && s < 1.099511627776e12f;      // 2^-40, 2^40
+        tab.col[c] = make_float4(m, s, plain ? 1.0f / s : 0.0f, (0.0f - m) / s);
+    }
+    uint32_t* sums = reinterpret_cast<uint32_t*>(dst);
+    {
+        uint32_t count = 0;
+        if (valid)
+        {
+#pragma unroll 15
+            for (int b = part; b < kBins; b += kParts) count += H.bin_count[b][z];
+        }
+        sums[threadIdx.x] = count;
     }
     __syncthreads();
-    const int pairs = kFeat / 16;
-    for (int t = threadIdx.x; t < kTcRows * pairs; t += kTcThreads)
+    if (part == 0 && valid)
     {
-        const int r8 = t & 7, rest = t >> 3, c2 = rest % pairs, g = rest / pairs, r = g * 8 + r8;
-        uint32_t packed[8];
-        const long row = row0 + r;
-        if (row < n)
-        {
-            const hw_lane_histogram& H = hist[row / kLane];
-            const int z = (int)(row % kLane);
+        uint32_t count = 0;
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
+        for (int q = 0; q < kParts; ++q) count += sums[q * kTcRows + r];
+        RowFeatures(count, H, st[row / kLane], z, rowInv[r], rowMean[r], rowVar[r]);
+    }
+    if (threadIdx.x < kFeat / 8)
+    {
+        uint32_t e[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+        {
+            const float4 c0 = tab.col[threadIdx.x * 8 + 2 * q], c1 = tab.col[threadIdx.x * 8 + 2 * q + 1];
+            e[q] = Pack2(__float2bfloat16_rn(c0.w), __float2bfloat16_rn(c1.w));
+        }
+        tab.empty[threadIdx.x] = make_uint4(e[0], e[1], e[2], e[3]);
+    }
+    __syncthreads();
+    const float inv = valid ? rowInv[r] : 0.0f;
+    uint16_t next[8];
+    auto load = [&](int c) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) next[j] = valid ? H.bin_count[c * 8 + j][z] : (uint16_t)0;
+    };
+    load(part);
+    for (int c = part; c < kBinChunks; c += kParts)
+    {
+        uint16_t n8[8];
+        uint32_t any = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+        {
+            n8[j] = next[j];
+            any |= n8[j];
+        }
+        if (c + kParts < kBinChunks) load(c + kParts);
+        uint4 w = tab.empty[c];
+        if (__any_sync(0xffffffffu, any != 0u))
+        {
+            uint32_t q4[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
             {
-                const int c = c2 * 16 + 2 * q;
-                const float f0 = FeatureValue(H, z, c, rowInv[r], rowMean[r], rowVar[r]);
-                const float f1 = FeatureValue(H, z, c + 1, rowInv[r], rowMean[r], rowVar[r]);
-                packed[q] = Pack2(__float2bfloat16_rn((f0 - mean[c]) / scale[c]),
-                                  __float2bfloat16_rn((f1 - mean[c + 1]) / scale[c + 1]));
+                const float f0 = sqrtf((float)n8[2 * q] * inv), f1 = sqrtf((float)n8[2 * q + 1] * inv);
+                q4[q] = Pack2(__float2bfloat16_rn(Standardise(f0, tab.col[c * 8 + 2 * q])),
+                              __float2bfloat16_rn(Standardise(f1, tab.col[c * 8 + 2 * q + 1])));
             }
+            w = make_uint4(q4[0], q4[1], q4[2], q4[3]);
         }
-        else
-        {
+        if (!valid) w = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(dst + CoreOffset(r, c, kFeat)) = w;
+    }
+    if (part == kParts - 1)
+    {
+        // the last chunk: bins 296..299, the two baseline features, padding
+        uint32_t q4[4];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) packed[q] = 0;
+        for (int q = 0; q < 4; ++q)
+        {
+            __nv_bfloat16 v[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+            {
+                const int c = kBinChunks * 8 + 2 * q + j;
+                const float f = valid ? FeatureValue(H, z, c, inv, rowMean[r], rowVar[r]) : 0.0f;
+                v[j] = __float2bfloat16_rn((f - tab.col[c].x) / tab.col[c].y);
+            }
+            q4[q] = valid ? Pack2(v[0], v[1]) : 0u;
         }
-        *reinterpret_cast<uint4*>(dst + CoreOffset(r, 2 * c2, kFeat)) =
-            make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        *reinterpret_cast<uint4*>(dst + CoreOffset(r, 2 * c2 + 1, kFeat)) =
-            make_uint4(packed[4], packed[5], packed[6], packed[7]);
+        *reinterpret_cast<uint4*>(dst + CoreOffset(r, kBinChunks, kFeat)) = make_uint4(q4[0], q4[1], q4[2], q4[3]);
     }
 }
 
@@ -492,8 +617,8 @@ __device__ __forceinline__ void HiddenEpilogue(uint32_t tbase, const float* __re
 #pragma unroll
             for (int j = 0; j < 4; ++j)
             {
-                const int c = c0 + q * 8 + 2 * j;
-                const float z0 = v[q * 8 + 2 * j] + bias[c], z1 = v[q * 8 + 2 * j + 1] + bias[c + 1];
+                const float2 b = __ldg(reinterpret_cast<const float2*>(bias + c0 + q * 8 + 2 * j));
+                const float z0 = v[q * 8 + 2 * j] + b.x, z1 = v[q * 8 + 2 * j + 1] + b.y;
                 p[j] = Pack2(__float2bfloat16_rn(GeluTanh(z0)), __float2bfloat16_rn(GeluTanh(z1)));
             }
             *reinterpret_cast<uint4*>(a + CoreOffset(r, c0 / 8 + q, kHidden)) = make_uint4(p[0], p[1], p[2], p[3]);
@@ -511,7 +636,7 @@ struct TcArgs
     const float* inScale;
     const float* outMean;
     const float* outScale;
-    const __nv_bfloat16* wb;
+    const __nv_bfloat16* wp;           // weight blocks in operand layout
     const float* master;
     float* out;                        // [n][32] standardised outputs, or
     float* proposal;                   // [lanes][15][64] EM starts
@@ -523,15 +648,18 @@ template <bool kHist>
 __global__ void __launch_bounds__(kTcThreads, 1) ForwardTcKernel(TcArgs p)
 {
     extern __shared__ __align__(1024) uint8_t tcSmem[];
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t bars[5];
     __shared__ uint32_t tmemSlot;
     __shared__ float rowInv[kTcRows], rowMean[kTcRows], rowVar[kTcRows];
+    __shared__ __align__(16) InputTable table;
     const long n = p.n;
-    const __nv_bfloat16* __restrict__ wb = p.wb;
+    const __nv_bfloat16* __restrict__ wp = p.wp;
     const float* __restrict__ master = p.master;
     uint8_t* A = tcSmem;
-    uint8_t* W = tcSmem + kTcA;
-    const uint32_t aAddr = SmemU32(A), wAddr = SmemU32(W), barAddr = SmemU32(&bar);
+    const uint32_t aAddr = SmemU32(A), wAddr = aAddr + kTcA;
+    // mbarriers: weights W1a then W2, W1b then W3, W1c; the first product's end; each layer's end
+    const uint32_t barL0 = SmemU32(&bars[0]), barL1 = SmemU32(&bars[1]), barL2 = SmemU32(&bars[2]);
+    const uint32_t barA = SmemU32(&bars[3]), barM = SmemU32(&bars[4]);
     const int warp = threadIdx.x >> 5;
     const long row0 = (long)blockIdx.x * kTcRows;
     // the output rows: warps 0..3, one row a thread
@@ -546,50 +674,72 @@ __global__ void __launch_bounds__(kTcThreads, 1) ForwardTcKernel(TcArgs p)
     }
     if (threadIdx.x == 0)
     {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(barAddr) : "memory");
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(barL0 + 8u * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        LoadWeights(wAddr, wp, kTcW1a, barL0);
+        LoadWeights(wAddr + kTcW1a, wp + kTcW1a / 2, kTcW1b, barL1);
     }
-    if (kHist) StageInputFromHist(p.hist, p.stats, row0, n, p.inMean, p.inScale, A, rowInv, rowMean, rowVar);
+    if (kHist) StageInputFromHist(p.hist, p.stats, row0, n, p.inMean, p.inScale, A, table, rowInv, rowMean, rowVar);
     else StageInput(p.feat, row0, n, p.inMean, p.inScale, A);
-    StageWeights(wb + kOffW1, kHidden / 2, kFeat, W);
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     PublishShared();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tbase = tmemSlot;
 
-    bool ok = true;
-    uint32_t parity = 0;
-    // layer 1, columns 0..127 then 128..255
-    for (int half = 0; half < 2 && ok; ++half)
+    // Layer 1: columns 0..127, 128..239 and, once the first product has read
+    // its weights, 240..255.  A wait that gives up issues nothing further, and
+    // the layer's wait below ends with its bound; a copy still in flight is
+    // waited for again (bounded) before the CTA ends.
+    uint32_t late = 0u, lateParity = 0u;      // a copy given up on: its mbarrier and phase
+    if (threadIdx.x == 0)
     {
-        if (half)
+        if (!WaitLoad(barL0, 0)) late = barL0;
+        else
         {
-            StageWeights(wb + kOffW1 + (size_t)(kHidden / 2) * kFeat, kHidden / 2, kFeat, W);
-            PublishShared();
+            MmaChain(tbase, aAddr, wAddr, kFeat, 128, barA);
+            if (!WaitLoad(barL1, 0)) late = barL1;
+            else
+            {
+                MmaIssue(tbase + 128, aAddr, wAddr + kTcW1a, kFeat, 112);
+                if (WaitLoad(barA, 0))
+                {
+                    LoadWeights(wAddr, wp + (kTcW1a + kTcW1b) / 2, kTcW1c, barL2);
+                    if (!WaitLoad(barL2, 0)) late = barL2;
+                    else MmaChain(tbase + 240, aAddr, wAddr, kFeat, 16, barM);
+                }
+            }
         }
-        if (threadIdx.x == 0) MmaChain(tbase + (uint32_t)(half * 128), aAddr, wAddr, kFeat, 128, barAddr);
-        ok = WaitMmas(barAddr, parity);
-        parity ^= 1;
     }
+    bool ok = WaitMmas(barM, 0);
     // layer 2
     if (ok)
     {
+        if (threadIdx.x == 0) LoadWeights(wAddr, wp + kPackW2, kTcW2, barL0);
         HiddenEpilogue(tbase, master + kOffB1, A);
-        StageWeights(wb + kOffW2, kHidden, kHidden, W);
         PublishShared();
-        if (threadIdx.x == 0) MmaChain(tbase, aAddr, wAddr, kHidden, kHidden, barAddr);
-        ok = WaitMmas(barAddr, parity);
-        parity ^= 1;
+        if (threadIdx.x == 0)
+        {
+            if (!WaitLoad(barL0, 1)) { late = barL0; lateParity = 1u; }
+            else MmaChain(tbase, aAddr, wAddr, kHidden, kHidden, barM);
+        }
+        ok = WaitMmas(barM, 1);
     }
     // layer 3
     if (ok)
     {
+        if (threadIdx.x == 0) LoadWeights(wAddr, wp + kPackW3, kTcW3, barL1);
         HiddenEpilogue(tbase, master + kOffB2, A);
-        StageWeights(wb + kOffW3, kOut, kHidden, W);
         PublishShared();
-        if (threadIdx.x == 0) MmaChain(tbase, aAddr, wAddr, kHidden, kOut, barAddr);
-        ok = WaitMmas(barAddr, parity);
+        if (threadIdx.x == 0)
+        {
+            if (!WaitLoad(barL1, 1)) { late = barL1; lateParity = 1u; }
+            else MmaChain(tbase, aAddr, wAddr, kHidden, kOut, barM);
+        }
+        ok = WaitMmas(barM, 0);
     }
+    if (late) WaitLoad(late, lateParity);
     if (ok && outWarp)
     {
         float v[32];
@@ -761,6 +911,7 @@ struct hw_learned_init
     float* m = nullptr;
     float* v = nullptr;
     __nv_bfloat16* wb = nullptr;   // BF16 copy of all parameters (the weight blocks are used)
+    __nv_bfloat16* wp = nullptr;   // its weight blocks in operand layout, for the forward pass
     float* norm = nullptr;     // input mean [304], input scale [304], output mean [32], output scale [32]
     __nv_bfloat16* X = nullptr;
     float* Z1 = nullptr;
@@ -781,7 +932,7 @@ struct hw_learned_init
 
     ~hw_learned_init()
     {
-        cudaFree(master); cudaFree(grad); cudaFree(m); cudaFree(v); cudaFree(wb); cudaFree(norm);
+        cudaFree(master); cudaFree(grad); cudaFree(m); cudaFree(v); cudaFree(wb); cudaFree(wp); cudaFree(norm);
         cudaFree(X); cudaFree(Z1); cudaFree(H1); cudaFree(Z2); cudaFree(H2); cudaFree(Y); cudaFree(T);
         cudaFree(dY); cudaFree(dA); cudaFree(loss); cudaFree(err);
     }
@@ -802,7 +953,7 @@ struct hw_learned_init
         a.inScale = InScale();
         a.outMean = OutMean();
         a.outScale = OutScale();
-        a.wb = wb;
+        a.wp = wp;
         a.master = master;
         a.err = err;
         ForwardTcKernel<kHist><<<(unsigned)((a.n + kTcRows - 1) / kTcRows), kTcThreads, kTcSmem, s>>>(a);
@@ -868,7 +1019,7 @@ int hw_learned_init_create(uint32_t max_batch, uint64_t seed, hw_learned_init** 
         if (rc == HW_OK) rc = Cuda(cudaMalloc((void**)p, count * sizeof(**p)), "hw_learned_init_create");
     };
     alloc(&h->master, kParams); alloc(&h->grad, kParams); alloc(&h->m, kParams); alloc(&h->v, kParams);
-    alloc(&h->wb, kParams); alloc(&h->norm, 2 * kFeat + 2 * kOut);
+    alloc(&h->wb, kParams); alloc(&h->wp, kPackAll); alloc(&h->norm, 2 * kFeat + 2 * kOut);
     alloc(&h->X, B * kFeat); alloc(&h->Z1, B * kHidden); alloc(&h->H1, B * kHidden); alloc(&h->Z2, B * kHidden);
     alloc(&h->H2, B * kHidden); alloc(&h->Y, B * kOut); alloc(&h->T, B * kOut); alloc(&h->dY, B * kOut);
     alloc(&h->dA, B * kHidden); alloc(&h->loss, 1); alloc(&h->err, 1);
@@ -897,6 +1048,7 @@ int hw_learned_init_create(uint32_t max_batch, uint64_t seed, hw_learned_init** 
     if (!rc)
     {
         ToBf16Kernel<<<Blocks((long)kParams), 256>>>(h->master, (int)kParams, h->wb);
+        PackWeightsKernel<<<Blocks((long)kPackAll), 256>>>(h->wb, h->wp);
         rc = Cuda(cudaDeviceSynchronize(), "hw_learned_init_create");
     }
     if (rc) { delete h; return rc; }
@@ -937,6 +1089,7 @@ int hw_learned_init_set_params(hw_learned_init* h, const float* host_params, con
         if (!rc)
         {
             ToBf16Kernel<<<Blocks((long)kParams), 256>>>(h->master, (int)kParams, h->wb);
+            PackWeightsKernel<<<Blocks((long)kPackAll), 256>>>(h->wb, h->wp);
             rc = Cuda(cudaDeviceSynchronize(), "set_params");
         }
     }
@@ -1048,6 +1201,7 @@ int hw_learned_init_train_step(hw_learned_init* h, const float* d_features, cons
         AdamWKernel<<<Blocks((long)g.count), 256, 0, s>>>(h->master + g.off, h->grad + g.off, h->m + g.off,
                                                           h->v + g.off, (int)g.count, lr, b1, b2, 1e-8f, g.wd, c1, c2,
                                                           h->wb + g.off);
+    PackWeightsKernel<<<Blocks((long)kPackAll), 256, 0, s>>>(h->wb, h->wp);
     return Cuda(cudaGetLastError(), "hw_learned_init_train_step");
 }
 
