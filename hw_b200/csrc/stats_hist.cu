@@ -267,7 +267,7 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
         // remainder underflows is far below 1 and keeps its sign).  A
         // division instead is twice the instructions and a branch a frame,
         // which kept the frames' chains from overlapping (reset, 8 chunks of
-        // 2048 lanes x 512 frames and read-out: 1490 -> 1295 us).  Chunks
+        // 2048 lanes x 512 frames and read-out: 1490 -> 1300 us).  Chunks
         // whose frames fill no whole batches, bin sizes out of range and a
         // classifier without two frames of history take the division.
         const float rcpBin = 1.0f / binSize;
@@ -336,9 +336,17 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
             aB[j] = __ldg(tr + (size_t)(S + j) * kLane);
         }
         int i = 0;
+        // Lines of both halves some batches ahead, one a thread (a frame of
+        // the lane is one line; the first 16 are loading already): a batch
+        // ahead in registers does not cover DRAM at 10 warps a SM (1300 ->
+        // 1200 us on the case above).
+        const int16_t* lines = tr - z + (size_t)((threadIdx.x & 16) ? S : 0) * kLane;
+        const int ahead = (int)(threadIdx.x & 15);
 #pragma unroll 1
         for (; i + 2 * kHistPairBatch <= S; i += 2 * kHistPairBatch)
         {
+            if ((i & 15) == 0 && threadIdx.x < 32 && i + 16 + ahead < S)
+                PrefetchL1(lines + (size_t)(i + 16 + ahead) * kLane);
 #pragma unroll
             for (int j = 0; j < kHistPairBatch; ++j)
             {
