@@ -5,12 +5,14 @@
 // uint8 ZMWs of one frame) lands at its ZMW's lane and frame of the pool's
 // chunk [lanes][frames][64].
 //
-// The host turns the chunk's packet table into copy segments -- the overlap
-// of one packet block with one lane, num_frames rows of 64 or 128 bytes with
-// the block's and the lane's row strides -- and one kernel moves them: a
-// 256-thread block per segment, 16-byte vector loads (streaming, the packets
-// are read once) and stores.  The copy is pure HBM traffic: every byte read
-// once and written once.
+// The chunk is cut into copy segments -- the overlap of one packet block with
+// one lane, num_frames rows of 64 or 128 bytes with the block's and the lane's
+// row strides -- and one kernel moves them: a 256-thread block per segment,
+// 16-byte vector loads (streaming, the packets are read once) and stores.  The
+// copy is pure HBM traffic: every byte read once and written once.  With few
+// packets that hold whole lanes the packet table itself is the kernel's
+// parameter and a block works out its segment; otherwise the host lists the
+// segments and uploads them.
 #include <algorithm>
 #include <string>
 #include <vector>
@@ -28,9 +30,8 @@ struct RepackSeg
     uint32_t srcStride, dstStride;  // bytes between rows
 };
 
-__global__ void __launch_bounds__(256) RepackKernel(const RepackSeg* segs)
+__device__ __forceinline__ void CopySegment(const RepackSeg& sg)
 {
-    const RepackSeg sg = segs[blockIdx.x];
     const uint32_t vpr = 1u << sg.vecsLog2;
     const uint32_t n = sg.rows << sg.vecsLog2;
     const char* src = reinterpret_cast<const char*>(sg.src);
@@ -41,6 +42,51 @@ __global__ void __launch_bounds__(256) RepackKernel(const RepackSeg* segs)
         const uint4 x = __ldcs(reinterpret_cast<const uint4*>(src + (size_t)row * sg.srcStride + col));
         *reinterpret_cast<uint4*>(dst + (size_t)row * sg.dstStride + col) = x;
     }
+}
+
+__global__ void __launch_bounds__(256) RepackKernel(const RepackSeg* segs) { CopySegment(segs[blockIdx.x]); }
+
+// A packet that starts at a lane and whose blocks hold whole lanes: segment i
+// of it is lane startLane + i.
+struct LanePacket
+{
+    uint64_t src;                       // device address of its data
+    uint32_t startLane, lanesPerBlock;
+    uint32_t frame0, rows;
+    uint32_t firstSeg;                  // segments of the packets before it
+    uint32_t blockBytes;                // of one frame of a block
+};
+
+constexpr int kMaxPackets = 64, kMaxPools = 64;      // 3 KB of the 4 KB parameters
+struct LanePackets
+{
+    LanePacket packet[kMaxPackets];
+    char* pool[kMaxPools];
+    int n;
+    uint32_t lanesPerPool, F, elem;
+};
+
+// A block's segment straight from the packets: no list to build, copy to the
+// device and wait for before the kernel (262,144 ZMWs x 512 int16 frames, 0.54
+// GB moved, in 8 packets: 112 -> 95 us, 5.7 TB/s; HBM bound).
+__global__ void __launch_bounds__(256) RepackPacketsKernel(const __grid_constant__ LanePackets t)
+{
+    int p = 0;
+    for (int step = kMaxPackets / 2; step; step /= 2)      // the last packet that starts at or before this segment
+        if (p + step < t.n && t.packet[p + step].firstSeg <= blockIdx.x) p += step;
+    const LanePacket& k = t.packet[p];
+    const uint32_t i = blockIdx.x - k.firstSeg, lane = k.startLane + i;
+    const uint32_t block = i / k.lanesPerBlock, inBlock = i % k.lanesPerBlock;
+    const uint32_t pool = lane / t.lanesPerPool, lip = lane % t.lanesPerPool;
+    const uint32_t row = kLane * t.elem;
+    RepackSeg s;
+    s.src = k.src + (uint64_t)block * k.rows * k.blockBytes + (uint64_t)inBlock * row;
+    s.dst = reinterpret_cast<uint64_t>(t.pool[pool]) + ((uint64_t)lip * t.F + k.frame0) * row;
+    s.rows = k.rows;
+    s.vecsLog2 = row == 128 ? 3 : 2;
+    s.srcStride = k.blockBytes;
+    s.dstStride = row;
+    CopySegment(s);
 }
 
 int Fail(int code, const std::string& msg) { return hwk::SetLastError(code, msg.c_str()); }
@@ -119,8 +165,11 @@ int hw_repack_chunk(hw_repacker* r, const hw_sensor_packet* packets, uint32_t n_
     const uint32_t e = r->elem;
     const uint32_t line = 64 / e;                 // ZMWs per cache line
     const uint64_t base = reinterpret_cast<uint64_t>(d_packet_data);
-    auto& segs = r->host;
-    segs.clear();
+    // The packets of whole lanes in the kernel's parameters while they fit.
+    LanePackets few;
+    few.n = 0;
+    bool byPacket = n_packets <= (uint32_t)kMaxPackets && r->pools <= (uint32_t)kMaxPools;
+    uint32_t fewSegs = 0;
     for (uint32_t i = 0; i < n_packets; ++i)
     {
         const hw_sensor_packet& p = packets[i];
@@ -134,6 +183,35 @@ int hw_repack_chunk(hw_repacker* r, const hw_sensor_packet* packets, uint32_t n_
             return Fail(HW_ERR_INVALID_ARG, "hw_repack_chunk: packet ZMWs outside the chip");
         if (p.start_zmw % line != 0)
             return Fail(HW_ERR_INVALID_ARG, "hw_repack_chunk: packet start must be cache-line aligned");
+        byPacket &= W % kLane == 0 && p.start_zmw % kLane == 0 && (uint64_t)W * e <= 0xffffffffull;
+        if (!byPacket) continue;
+        const uint32_t lane0 = p.start_zmw / kLane, lanes = p.num_blocks * (W / kLane);
+        for (uint32_t q = lane0 / r->lanesPerPool; lanes && q <= (lane0 + lanes - 1) / r->lanesPerPool; ++q)
+            if (!d_pool_chunks[q]) return Fail(HW_ERR_INVALID_ARG, "hw_repack_chunk: NULL pool chunk");
+        if (lanes == 0) continue;
+        few.packet[few.n++] = LanePacket{base + p.data_offset, lane0, W / kLane,
+                                         (uint32_t)(p.start_frame - chunk_first_frame), N, fewSegs, W * e};
+        fewSegs += lanes;
+    }
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    if (byPacket)
+    {
+        if (fewSegs == 0) return HW_OK;
+        for (uint32_t q = 0; q < r->pools; ++q) few.pool[q] = static_cast<char*>(d_pool_chunks[q]);
+        few.lanesPerPool = r->lanesPerPool;
+        few.F = r->F;
+        few.elem = e;
+        RepackPacketsKernel<<<fewSegs, 256, 0, s>>>(few);
+        const cudaError_t pe = cudaGetLastError();
+        if (pe != cudaSuccess) return Fail(HW_ERR_CUDA, std::string("hw_repack_chunk: ") + cudaGetErrorString(pe));
+        return HW_OK;
+    }
+    auto& segs = r->host;
+    segs.clear();
+    for (uint32_t i = 0; i < n_packets; ++i)
+    {
+        const hw_sensor_packet& p = packets[i];
+        const uint32_t W = p.block_width, N = p.num_frames;
         const uint32_t frame0 = (uint32_t)(p.start_frame - chunk_first_frame);
         for (uint32_t b = 0; b < p.num_blocks; ++b)
         {
@@ -160,7 +238,6 @@ int hw_repack_chunk(hw_repacker* r, const hw_sensor_packet* packets, uint32_t n_
         }
     }
     if (segs.empty()) return HW_OK;
-    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     const int b = (int)(r->calls & 1);
     // the call that last used staging buffer b must have copied it already
     if (r->inFlight[b] && cudaEventSynchronize(r->ev[b]) != cudaSuccess)

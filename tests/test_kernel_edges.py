@@ -150,3 +150,34 @@ def test_baseline_ranges(F, pedestal, sensitivity, extreme):
             out += b.baseline(np.ascontiguousarray(tr[:, c * F:(c + 1) * F]), c * F)
         return out
     _both(cfg, lanes, F, call)
+
+
+@pytest.mark.parametrize("encoding", [0, 1])
+@pytest.mark.parametrize("lanes_per_pool,packet_blocks,width", [(16, 2, 128), (16, 1, 128), (2, 4, 64), (1, 4, 64),
+                                                                (7, 64, 64), (128, 5, 192)])
+def test_repack_paths(lanes_per_pool, packet_blocks, width, encoding):
+    """Up to 64 packets and pools go to the kernel, more through the list:
+    both sides of the line (64 or 128 packets, 64 or 128 pools), blocks of one
+    to three lanes, a packet without blocks, a missing pool."""
+    import torch
+    from hw_b200 import filters as Fl
+    from hw_b200.native import HwError
+    import test_repack as R
+    num_zmw, F = 128 * 64, 64
+    table, data = R.make_chunk(num_zmw, 0, F, 64, packet_blocks, width, encoding)
+    none = table[:1].copy()
+    none["num_blocks"] = 0
+    table = np.concatenate([table[:1], none, table[1:]])
+    rp = Fl.Repacker(num_zmw, lanes_per_pool, F, "int16" if encoding == 0 else "uint8")
+    chunks = rp.new_chunks()
+    d = torch.from_numpy(data.copy()).cuda()
+    rp(table, d, 0, chunks)
+    want = R.oracle_repack(num_zmw, lanes_per_pool, F, encoding, table, data, 0)
+    for got, w in zip(chunks, want):
+        assert np.array_equal(got.cpu().numpy(), w)
+
+    class Missing:
+        def data_ptr(self):
+            return 0
+    with pytest.raises(HwError):
+        rp(table, d, 0, chunks[:-1] + [Missing()])
