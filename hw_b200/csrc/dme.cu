@@ -539,8 +539,9 @@ __device__ __noinline__ void EmEStepGeneric(EmStepIo& io)
 // Bound by the FMA pipe (60%) and the dependent chain of a boundary; one thread
 // a ZMW, modes 0/1 and 2/3 as packed pairs.  A 4096-lane estimate took 18.5 ms
 // with the general form alone (84,900 thread instructions a ZMW and iteration)
-// and takes 11.5 ms (41,000); 37 lanes 3.24 -> 1.51 ms.  8 blocks a SM, where
-// nothing spills: 10 blocks with spills 12.3 ms, 7 blocks 11.5 ms.
+// and takes 10.8 ms (41,000); 37 lanes 3.35 -> 1.50 ms.  8 blocks a SM, where
+// nothing spills: before the M-step's last change 11.5 ms, 10 blocks with
+// spills 12.3 ms, 7 blocks 11.5 ms.
 template <bool kFull = true>
 __device__ __forceinline__ float EmEStep(const KParams& k, const EmHist& h, const EmVars& v, const EmReg& r,
                                          float* bpS, float* tau0S, float* facS, float ci[5], float mom1[5],
@@ -760,9 +761,12 @@ __device__ __forceinline__ void EmMStep(const KParams& k, const EmHist& h, const
             bpj = bpS[(size_t)j0 * kLane + z];
             t0j = tau0S[(size_t)j0 * kLane + z];
         }
-        // four bins' values are loaded together (memory latency bounds this
-        // pass); past the last bin the last one's are loaded and not used
-        constexpr int kB = 4;
+        // Sixteen bins' values are loaded together: the scratch of the lanes
+        // in flight is larger than L2, so memory latency bounds this pass
+        // (24% of an estimate with four at a time; a 4096-lane estimate 11.47
+        // -> 10.77 ms, 10.84 with eight).  Past the last bin the last one's
+        // are loaded and not used.
+        constexpr int kB = 16;
         float jf = (float)j0;
         for (int jj = j0; jj < j1; jj += kB)
         {
