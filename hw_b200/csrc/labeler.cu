@@ -321,7 +321,7 @@ constexpr int kGenericShift = 3;
 // a value needs one maximum and a decision one subtraction (FMA pipe) and one
 // funnel shift that appends the sign to the traceback word: with compares and
 // selects instead (422 thread instructions a ZMW-frame over the kernel, 68% of
-// the ALU pipe) 4096 lanes x 512 frames took 2145 us; now 299, 55% and 1560 us.
+// the ALU pipe) 4096 lanes x 512 frames took 2145 us; now 293, 55% and 1560 us.
 // Issue and ALU latency bound it now (65% of issue slots at 5 warps a
 // scheduler, the most that 96 registers allow; 4 and 6 warps measured 1659 and
 // 1616 us).
