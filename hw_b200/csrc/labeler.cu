@@ -10,9 +10,10 @@
 //   2. runs the max-plus Viterbi over 24 latent + F-8 chunk frames + 16
 //      look-ahead frames in fp32 with the reference's operation order and
 //      tie rule (a later source state wins ties);
-//   3. stores one 28-bit traceback word per frame: the arg-max source of each
-//      destination row, coded in 4 bits for the 9-way rows (baseline and the
-//      four pulse-up rows) and 1 bit for the 2-way rows (full and down);
+//   3. stores one traceback word per frame: the generic rows code the arg-max
+//      source of each destination row, 4 bits for the 9-way rows (baseline and
+//      the four pulse-up rows) and 1 bit for the 2-way rows (full and down);
+//      the grouped rows the decisions that lead to it (GroupedStep);
 //   4. back-propagates the normalised end-state probabilities 16 frames,
 //      picks the anchor state and traces back F frames.
 // Traceback words live in a global scratch laid out [lane][frame][zmw] so
