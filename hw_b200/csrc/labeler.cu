@@ -314,7 +314,8 @@ constexpr int kGenericShift = 3;
 // m_G and its position are found once for the five rows, by two rounds of
 // pairwise comparisons, and a frame where one of a group's comparisons is
 // closer than 2^-21 (|score| + |t| + |m_G|) over all rows, or whose scorer is
-// not `ordinary`, takes the generic rows.
+// not `ordinary` or whose log-likelihoods came with a NaN (bad), takes the
+// generic rows.
 //
 // Every decision "the later candidate is at least the earlier one" is the sign
 // of their difference: 0 for yes (also for equal values and for two -inf,
@@ -679,7 +680,14 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
 #pragma unroll
             for (int i = 0; i < kStates; ++i) anchorLL(i) = ll.Get(i);
         }
-        const bool bad = !sc.ordinary;
+        // A NaN (or +inf) that the old model's scores left in the
+        // log-likelihoods is kept by the generic rows' comparisons and would
+        // be dropped by GroupedStep's maxima: the new model's segment takes
+        // the generic rows then, however ordinary the model.
+        float sum = ll.s0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sum += add_rn(ll.p[q].x, ll.p[q].y);
+        const bool bad = !sc.ordinary | !(sum < __int_as_float(0x7f800000));
         uint32_t roiWord = ~roiw((lf + 2) >> 5) << ((lf + 2) & 31);
         int16_t x0 = __ldg(src + (size_t)lf * kLane);
         int16_t x1 = __ldg(src + (size_t)(lf + 1 < end ? lf + 1 : lf) * kLane);

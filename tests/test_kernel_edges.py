@@ -131,6 +131,36 @@ def test_label_paths(kind, F):
     _both(cfg, lanes, F, call)
 
 
+@pytest.mark.parametrize("kind", ["zero_var", "zero_analog_var", "nan_var", "nan_mean", "inf_var"])
+@pytest.mark.parametrize("F", [48, 512])
+def test_label_model_recovers(kind, F):
+    """A ZMW whose model scores NaN in one chunk and is ordinary in the next:
+    the next chunk's latent frames still take the old model, and the NaN they
+    leave in the log-likelihoods is the generic rows' to carry."""
+    lanes = 2
+    good, bad = _models(lanes), _models(lanes)
+    odd = slice(1, None, 3)
+    if kind == "zero_var":
+        bad["baseline"]["vars"][:, odd] = 0
+    elif kind == "zero_analog_var":
+        bad["analogs"]["vars"][:, 0, odd] = 0
+    elif kind == "nan_var":
+        bad["analogs"]["vars"][:, 1, odd] = 0x7e00
+    elif kind == "nan_mean":
+        bad["analogs"]["means"][:, 2, odd] = 0x7e00
+    elif kind == "inf_var":
+        bad["baseline"]["vars"][:, odd] = 0x7c00
+        bad["analogs"]["vars"][:, 3, odd] = 0x7c00
+    tr = synth.traces(lanes, 6 * F, seed=F, gain_sigma=0.2, empty_fraction=0.1, baseline=0.0)
+
+    def call(b):
+        out = []
+        for c in range(6):
+            out += b.label(np.ascontiguousarray(tr[:, c * F:(c + 1) * F]), good if c % 2 else bad)
+        return out
+    _both(workloads.small_config(), lanes, F, call)
+
+
 @pytest.mark.parametrize("F", [48, 512])
 @pytest.mark.parametrize("pedestal,sensitivity,extreme", [(0, 1.0, False), (13, 1.9, False), (-32768, 0.01, True),
                                                           (32767, 62.0, True), (5, 100.0, True), (0, 3.0e7, False)])
