@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(128) GemmKernel(const TA* __restrict__ A, long
 }
 
 // ---- Fused forward pass on the sm_100 tensor cores (tcgen05 + TMEM) ------------
-// One CTA of 128 threads per 128 rows runs all three layers: the
+// One CTA of 512 threads per 128 rows runs all three layers: the
 // standardised BF16 input tile and each layer's BF16 weights are staged in
 // shared memory as canonical K-major core matrices (8 rows x 16 bytes,
 // no swizzle: rows 16 bytes apart, the next 8-column group 128 bytes on,
@@ -293,8 +293,10 @@ __global__ void __launch_bounds__(128) GemmKernel(const TA* __restrict__ A, long
 // tile, beside the second product; W2 and W3 beside the epilogues.  Rounding
 // points are those of the mma.sync path (BF16 inputs and activations, FP32
 // accumulation and epilogue); only the order of the FP32 accumulation differs.
-// Every wait on an mbarrier is bounded: past about a second the CTA writes NaN
-// rows (a proposal the DME's fallback test rejects), sets *err and returns.
+// Every wait on an mbarrier is bounded by one deadline of the CTA (kTcWaitCycles
+// after its input is staged, about a second): past it the CTA waits, bounded again, for
+// the copies and products it has in flight, writes NaN rows (a proposal the
+// DME's fallback test rejects), sets *err and returns.
 //
 // Bound by the scalar work of a tile (features, standardisation, GELU): one CTA
 // a SM by shared memory, the products a few us of the tile.  262,144 rows from
@@ -344,16 +346,24 @@ __device__ __forceinline__ bool MbarTryWait(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
-// All threads: wait for the MMAs committed to `bar` (phase `parity`); false
-// (for every thread) when any thread gave up.
-__device__ __forceinline__ bool WaitMmas(uint32_t bar, uint32_t parity)
+constexpr long long kTcWaitCycles = 2000000000ll;
+
+// Wait for phase `parity` of `bar`; false when the clock passes `end` first.
+__device__ __forceinline__ bool WaitBar(uint32_t bar, uint32_t parity, long long end)
 {
-    const long long t0 = clock64();
-    bool ok = false;
+    bool ok;
     while (!(ok = MbarTryWait(bar, parity)))
-        if (clock64() - t0 > 4000000000ll) break;
+        if (clock64() > end) break;
+    return ok;
+}
+
+// All threads: wait for the MMAs committed to `bar` (phase `parity`); false
+// (for every thread) when any thread gave up or came with good = false.
+__device__ __forceinline__ bool WaitMmas(uint32_t bar, uint32_t parity, long long end, bool good)
+{
+    const bool ok = WaitBar(bar, parity, end);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    return !__syncthreads_or(!ok);
+    return !__syncthreads_or(!ok | !good);
 }
 
 // Issued by one thread: D[tmem] (+)= A (128 x K) . B (N x K)^T over K / 16 steps.
@@ -365,10 +375,9 @@ __device__ __forceinline__ void MmaIssue(uint32_t d, uint32_t a, uint32_t b, int
         UmmaBf16(d, UmmaDesc(a + s * 256u, 128u, sbo), UmmaDesc(b + s * 256u, 128u, sbo), idesc, s > 0);
 }
 
-// The same, and `bar` completes when these and all earlier products have.
-__device__ __forceinline__ void MmaChain(uint32_t d, uint32_t a, uint32_t b, int k, int n, uint32_t bar)
+// `bar` completes when all products issued before have.
+__device__ __forceinline__ void MmaCommit(uint32_t bar)
 {
-    MmaIssue(d, a, b, k, n);
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar)
                  : "memory");
 }
@@ -400,15 +409,6 @@ __device__ __forceinline__ void LoadWeights(uint32_t dst, const __nv_bfloat16* s
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-
-// One thread: bounded wait for phase `parity` of `bar`.
-__device__ __forceinline__ bool WaitLoad(uint32_t bar, uint32_t parity)
-{
-    const long long t0 = clock64();
-    while (!MbarTryWait(bar, parity))
-        if (clock64() - t0 > 4000000000ll) return MbarTryWait(bar, parity);
-    return true;
 }
 
 // The standardised input tile (rows past n are 0), as InputKernel rounds it.
@@ -645,14 +645,40 @@ struct TcArgs
     float* out;                        // [n][32] standardised outputs, or
     float* proposal;                   // [lanes][15][64] EM starts
     int* err;
+    long long waitCycles;              // the CTA's deadline
+    int withhold;                      // with kTest: the copy or commit (TcStep) that is left out
 };
 
+// mbarriers: weights W1a then W2, W1b then W3, W1c; the first product's end; each layer's end; all
+// products' end after a wait that gave up
+enum TcBar { kBarL0, kBarL1, kBarL2, kBarA, kBarM, kBarEnd, kTcBars };
+// copies and commits in their order
+enum TcStep { kStepW1a, kStepW1b, kStepA, kStepW1c, kStepM1, kStepW2, kStepM2, kStepW3, kStepM3, kTcSteps };
+
+// What a thread that gave up may still have in flight: bit b for phase 0 of
+// mbarrier b, bit 8 + b for phase 1.
+constexpr uint32_t TcOpen(int b, uint32_t parity = 0u) { return 1u << (b + 8 * (int)parity); }
+
+// The issuing thread after a wait gave up: a copy left behind could land in the
+// next CTA's shared memory, a product in its tensor memory, so it waits for
+// both, bounded again.  The commit covers every product issued, committed
+// before or not.
+__device__ __noinline__ void DrainLate(uint32_t barBase, uint32_t late, long long waitCycles)
+{
+    MmaCommit(barBase + 8u * kBarEnd);
+    const long long end = clock64() + waitCycles;
+    WaitBar(barBase + 8u * kBarEnd, 0u, end);
+    for (uint32_t i = 0; i < 16u; ++i)
+        if ((late >> i) & 1u) WaitBar(barBase + 8u * (i & 7u), i >> 3, end);
+}
+
 // kHist: features from the histograms and the proposal written directly.
-template <bool kHist>
+// kTest: p.withhold leaves out a copy or commit (hw_learned_init_set_wait_limit).
+template <bool kHist, bool kTest>
 __global__ void __launch_bounds__(kTcThreads, 1) ForwardTcKernel(TcArgs p)
 {
     extern __shared__ __align__(1024) uint8_t tcSmem[];
-    __shared__ __align__(8) uint64_t bars[5];
+    __shared__ __align__(8) uint64_t bars[kTcBars];
     __shared__ uint32_t tmemSlot;
     __shared__ float rowInv[kTcRows], rowMean[kTcRows], rowVar[kTcRows];
     __shared__ __align__(16) InputTable table;
@@ -661,9 +687,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) ForwardTcKernel(TcArgs p)
     const float* __restrict__ master = p.master;
     uint8_t* A = tcSmem;
     const uint32_t aAddr = SmemU32(A), wAddr = aAddr + kTcA;
-    // mbarriers: weights W1a then W2, W1b then W3, W1c; the first product's end; each layer's end
-    const uint32_t barL0 = SmemU32(&bars[0]), barL1 = SmemU32(&bars[1]), barL2 = SmemU32(&bars[2]);
-    const uint32_t barA = SmemU32(&bars[3]), barM = SmemU32(&bars[4]);
+    const uint32_t barBase = SmemU32(bars);
+    auto bar = [&](int b) -> uint32_t { return barBase + 8u * (uint32_t)b; };
+    auto load = [&](int step, int b, uint32_t dst, const __nv_bfloat16* src, uint32_t bytes) {
+        if (!kTest || step != p.withhold) LoadWeights(dst, src, bytes, bar(b));
+    };
+    auto commit = [&](int step, int b) {
+        if (!kTest || step != p.withhold) MmaCommit(bar(b));
+    };
     const int warp = threadIdx.x >> 5;
     const long row0 = (long)blockIdx.x * kTcRows;
     // the output rows: warps 0..3, one row a thread
@@ -679,71 +710,91 @@ __global__ void __launch_bounds__(kTcThreads, 1) ForwardTcKernel(TcArgs p)
     if (threadIdx.x == 0)
     {
 #pragma unroll
-        for (int i = 0; i < 5; ++i)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(barL0 + 8u * i) : "memory");
+        for (int i = 0; i < kTcBars; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar(i)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        LoadWeights(wAddr, wp, kTcW1a, barL0);
-        LoadWeights(wAddr + kTcW1a, wp + kTcW1a / 2, kTcW1b, barL1);
+        load(kStepW1a, kBarL0, wAddr, wp, kTcW1a);
+        load(kStepW1b, kBarL1, wAddr + kTcW1a, wp + kTcW1a / 2, kTcW1b);
     }
     if (kHist) StageInputFromHist(p.hist, p.stats, row0, n, p.inMean, p.inScale, A, table, rowInv, rowMean, rowVar);
     else StageInput(p.feat, row0, n, p.inMean, p.inScale, A);
     PublishShared();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tbase = tmemSlot;
+    const long long end = clock64() + p.waitCycles;
 
     // Layer 1: columns 0..127, 128..239 and, once the first product has read
-    // its weights, 240..255.  A wait that gives up issues nothing further, and
-    // the layer's wait below ends with its bound; a copy still in flight is
-    // waited for again (bounded) before the CTA ends.
-    uint32_t late = 0u, lateParity = 0u;      // a copy given up on: its mbarrier and phase
+    // its weights, 240..255.  A wait that gives up issues nothing further and
+    // notes what may be in flight (late); the layer's wait below then ends at
+    // once, its deadline has passed too.
+    uint32_t late = 0u, layerEnd = TcOpen(kBarM);
     if (threadIdx.x == 0)
     {
-        if (!WaitLoad(barL0, 0)) late = barL0;
+        if (!WaitBar(bar(kBarL0), 0u, end)) late = TcOpen(kBarL0) | TcOpen(kBarL1);
         else
         {
-            MmaChain(tbase, aAddr, wAddr, kFeat, 128, barA);
-            if (!WaitLoad(barL1, 0)) late = barL1;
+            MmaIssue(tbase, aAddr, wAddr, kFeat, 128);
+            commit(kStepA, kBarA);
+            if (!WaitBar(bar(kBarL1), 0u, end)) late = TcOpen(kBarL1) | TcOpen(kBarA);
             else
             {
                 MmaIssue(tbase + 128, aAddr, wAddr + kTcW1a, kFeat, 112);
-                if (WaitLoad(barA, 0))
+                if (!WaitBar(bar(kBarA), 0u, end)) late = TcOpen(kBarA);
+                else
                 {
-                    LoadWeights(wAddr, wp + (kTcW1a + kTcW1b) / 2, kTcW1c, barL2);
-                    if (!WaitLoad(barL2, 0)) late = barL2;
-                    else MmaChain(tbase + 240, aAddr, wAddr, kFeat, 16, barM);
+                    load(kStepW1c, kBarL2, wAddr, wp + (kTcW1a + kTcW1b) / 2, kTcW1c);
+                    if (!WaitBar(bar(kBarL2), 0u, end)) late = TcOpen(kBarL2);
+                    else
+                    {
+                        MmaIssue(tbase + 240, aAddr, wAddr, kFeat, 16);
+                        commit(kStepM1, kBarM);
+                    }
                 }
             }
         }
     }
-    bool ok = WaitMmas(barM, 0);
+    bool ok = WaitMmas(bar(kBarM), 0u, end, late == 0u);
     // layer 2
     if (ok)
     {
-        if (threadIdx.x == 0) LoadWeights(wAddr, wp + kPackW2, kTcW2, barL0);
+        if (threadIdx.x == 0) load(kStepW2, kBarL0, wAddr, wp + kPackW2, kTcW2);
         HiddenEpilogue(tbase, master + kOffB1, A);
         PublishShared();
         if (threadIdx.x == 0)
         {
-            if (!WaitLoad(barL0, 1)) { late = barL0; lateParity = 1u; }
-            else MmaChain(tbase, aAddr, wAddr, kHidden, kHidden, barM);
+            layerEnd = TcOpen(kBarM, 1u);
+            if (!WaitBar(bar(kBarL0), 1u, end)) late = TcOpen(kBarL0, 1u);
+            else
+            {
+                MmaIssue(tbase, aAddr, wAddr, kHidden, kHidden);
+                commit(kStepM2, kBarM);
+            }
         }
-        ok = WaitMmas(barM, 1);
+        ok = WaitMmas(bar(kBarM), 1u, end, late == 0u);
     }
     // layer 3
     if (ok)
     {
-        if (threadIdx.x == 0) LoadWeights(wAddr, wp + kPackW3, kTcW3, barL1);
+        if (threadIdx.x == 0) load(kStepW3, kBarL1, wAddr, wp + kPackW3, kTcW3);
         HiddenEpilogue(tbase, master + kOffB2, A);
         PublishShared();
         if (threadIdx.x == 0)
         {
-            if (!WaitLoad(barL1, 1)) { late = barL1; lateParity = 1u; }
-            else MmaChain(tbase, aAddr, wAddr, kHidden, kOut, barM);
+            layerEnd = TcOpen(kBarM);
+            if (!WaitBar(bar(kBarL1), 1u, end)) late = TcOpen(kBarL1, 1u);
+            else
+            {
+                MmaIssue(tbase, aAddr, wAddr, kHidden, kOut);
+                commit(kStepM3, kBarM);
+            }
         }
-        ok = WaitMmas(barM, 0);
+        ok = WaitMmas(bar(kBarM), 0u, end, late == 0u);
     }
-    if (late) WaitLoad(late, lateParity);
+    if (!ok && threadIdx.x == 0)
+    {
+        DrainLate(barBase, late ? late : layerEnd, p.waitCycles);
+    }
     if (ok && outWarp)
     {
         float v[32];
@@ -928,6 +979,8 @@ struct hw_learned_init
     float* dA = nullptr;       // [maxBatch][256] hidden gradient
     float* loss = nullptr;
     int* err = nullptr;        // set by the tensor-core forward pass when a wait timed out
+    long long waitCycles = hwk::kTcWaitCycles;
+    int withhold = -1;
 
     float* InMean() const { return norm; }
     float* InScale() const { return norm + kFeat; }
@@ -945,11 +998,18 @@ struct hw_learned_init
     template <bool kHist>
     int LaunchTc(TcArgs a, cudaStream_t s, const char* where)
     {
+        if (withhold >= 0) return LaunchTc<kHist, true>(a, s, where);
+        return LaunchTc<kHist, false>(a, s, where);
+    }
+
+    template <bool kHist, bool kTest>
+    int LaunchTc(TcArgs a, cudaStream_t s, const char* where)
+    {
         static bool attr = false;
         if (!attr)
         {
-            const int rc = Cuda(cudaFuncSetAttribute(ForwardTcKernel<kHist>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     kTcSmem), where);
+            const int rc = Cuda(cudaFuncSetAttribute(ForwardTcKernel<kHist, kTest>,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem), where);
             if (rc) return rc;
             attr = true;
         }
@@ -960,7 +1020,9 @@ struct hw_learned_init
         a.wp = wp;
         a.master = master;
         a.err = err;
-        ForwardTcKernel<kHist><<<(unsigned)((a.n + kTcRows - 1) / kTcRows), kTcThreads, kTcSmem, s>>>(a);
+        a.waitCycles = waitCycles;
+        a.withhold = withhold;
+        ForwardTcKernel<kHist, kTest><<<(unsigned)((a.n + kTcRows - 1) / kTcRows), kTcThreads, kTcSmem, s>>>(a);
         return Cuda(cudaGetLastError(), where);
     }
 
@@ -1153,6 +1215,15 @@ int hw_learned_init_forward_status(hw_learned_init* h)
         cudaMemset(h->err, 0, sizeof(int));
         return SetLastError(e, "hw_learned_init_forward: a tensor-core wait timed out (rows written as NaN)");
     }
+    return HW_OK;
+}
+
+int hw_learned_init_set_wait_limit(hw_learned_init* h, uint64_t cycles, int32_t withhold)
+{
+    if (!h || cycles == 0 || cycles > (uint64_t)kTcWaitCycles || withhold < -1 || withhold >= kTcSteps)
+        return SetLastError(HW_ERR_INVALID_ARG, "hw_learned_init_set_wait_limit: bad argument");
+    h->waitCycles = (long long)cycles;
+    h->withhold = withhold;
     return HW_OK;
 }
 

@@ -129,6 +129,7 @@ def lib():
         "hw_learned_init_targets": ([PCFG, u32, vp, vp, vp, vp], C.c_int),
         "hw_learned_init_forward": ([vp, vp, u32, vp, vp], C.c_int),
         "hw_learned_init_forward_status": ([vp], C.c_int),
+        "hw_learned_init_set_wait_limit": ([vp, C.c_uint64, C.c_int32], C.c_int),
         "hw_learned_init_propose": ([vp, u32, vp, vp, vp, vp], C.c_int),
         "hw_learned_init_proposal": ([vp, u32, vp, vp, vp, vp], C.c_int),
         "hw_learned_init_gradients": ([vp, vp, vp, vp, u32, vp, C.POINTER(C.c_float), vp], C.c_int),

@@ -465,6 +465,11 @@ int hw_learned_init_forward(hw_learned_init* h, const float* d_features, uint32_
  * since the last call gave up a bounded tensor-core wait -- its rows were
  * written as NaN, which the learned start's fallback test rejects. */
 int hw_learned_init_forward_status(hw_learned_init* h);
+/* The bound on a tile's waits, in clock cycles from its staged input (default
+ * and largest 2e9, about a second).  withhold >= 0 leaves out one copy or commit
+ * of each tile (0 to 8, in their order), so that a wait runs out -- for tests
+ * of the bounded wait only; -1 for normal use. */
+int hw_learned_init_set_wait_limit(hw_learned_init* h, uint64_t cycles, int32_t withhold);
 /* Features, forward pass and EM start of lanes * 64 ZMWs in one launch:
  * equal to hw_learned_init_features -> hw_learned_init_forward ->
  * hw_learned_init_proposal without the [n][304] and [n][32] intermediates.

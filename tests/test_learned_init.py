@@ -102,6 +102,34 @@ def test_fused_proposal_equals_the_three_steps():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("step", range(9))
+def test_forward_gives_up_at_every_wait_and_recovers(step):
+    """Each weight copy and each commit of a tile left out in turn (a test
+    hook): the wait behind it runs out after about a millisecond, every row is
+    NaN and the status HW_ERR_TIMEOUT, several waves of tiles over.  What the
+    tiles had in flight is waited for, so the next pass gives the bits of the
+    first."""
+    from hw_b200 import learned_init as L, native
+    rng = np.random.default_rng(3)
+    net = L.Network(max_batch=256, seed=3)
+    p, norm = _random_net(rng)
+    net.set(p, norm)
+    feat = _dev(rng.standard_normal((128 * 400 + 37, R.FEAT)).astype(np.float32))
+    want = net.forward(feat).cpu().numpy()
+    net.forward_status()
+    lib = native.lib()
+    assert lib.hw_learned_init_set_wait_limit(net._h, 2000000, step) == 0
+    got = net.forward(feat).cpu().numpy()
+    with pytest.raises(native.HwError) as err:
+        net.forward_status()
+    assert err.value.code == 7 and np.isnan(got).all()
+    assert lib.hw_learned_init_set_wait_limit(net._h, 2000000000, -1) == 0
+    again = net.forward(feat).cpu().numpy()
+    net.forward_status()
+    assert np.isfinite(want).all() and again.tobytes() == want.tobytes()
+
+
+@pytest.mark.gpu
 def test_forward_and_gradients_match_reference():
     """BF16 tensor-core forward and backward against the CPU reference with
     the same BF16 rounding points; they differ only by FP32 accumulation order
