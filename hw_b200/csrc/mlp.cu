@@ -1002,17 +1002,25 @@ struct hw_learned_init
         return LaunchTc<kHist, false>(a, s, where);
     }
 
+    // The forward kernels' shared memory, an attribute of the current device
+    // (set for every handle: another handle may live on another device).
+    static cudaError_t AllowTcSmem()
+    {
+        cudaError_t e = cudaSuccess;
+        auto allow = [&](auto* kernel) {
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+        };
+        allow(ForwardTcKernel<false, false>);
+        allow(ForwardTcKernel<false, true>);
+        allow(ForwardTcKernel<true, false>);
+        allow(ForwardTcKernel<true, true>);
+        return e;
+    }
+
     template <bool kHist, bool kTest>
     int LaunchTc(TcArgs a, cudaStream_t s, const char* where)
     {
-        static bool attr = false;
-        if (!attr)
-        {
-            const int rc = Cuda(cudaFuncSetAttribute(ForwardTcKernel<kHist, kTest>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem), where);
-            if (rc) return rc;
-            attr = true;
-        }
         a.inMean = InMean();
         a.inScale = InScale();
         a.outMean = OutMean();
@@ -1090,6 +1098,7 @@ int hw_learned_init_create(uint32_t max_batch, uint64_t seed, hw_learned_init** 
     alloc(&h->H2, B * kHidden); alloc(&h->Y, B * kOut); alloc(&h->T, B * kOut); alloc(&h->dY, B * kOut);
     alloc(&h->dA, B * kHidden); alloc(&h->loss, 1); alloc(&h->err, 1);
     if (!rc) rc = Cuda(cudaMemset(h->err, 0, sizeof(int)), "hw_learned_init_create");
+    if (!rc) rc = Cuda(hw_learned_init::AllowTcSmem(), "hw_learned_init_create");
     if (rc) { delete h; return rc; }
     // He-normal weights (std sqrt(2 / fan_in)) from a seeded host generator,
     // zero biases, zero rows for the unused outputs.
