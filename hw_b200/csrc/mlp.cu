@@ -168,9 +168,20 @@ template <typename T> __device__ __forceinline__ __nv_bfloat16 ToBf16(T v);
 template <> __device__ __forceinline__ __nv_bfloat16 ToBf16<float>(float v) { return __float2bfloat16_rn(v); }
 template <> __device__ __forceinline__ __nv_bfloat16 ToBf16<__nv_bfloat16>(__nv_bfloat16 v) { return v; }
 
-// 0.5 x (1 + tanh(u)) = x / (1 + exp(-2 u)), u = k0 (x + k1 x^3): no
-// cancellation where the tanh is near -1, and a third of the instructions.
 __device__ __forceinline__ float GeluTanh(float x)
+{
+    const float k0 = 0.7978845608028654f, k1 = 0.044715f;
+    return 0.5f * x * (1.0f + tanhf(k0 * (x + k1 * x * x * x)));
+}
+
+// The same as x / (1 + exp(-2 u)), u = k0 (x + k1 x^3), a third of the
+// instructions, for the fused forward pass, which is bound by them.  Training
+// keeps the form above: its time does not depend on it, and a run's network
+// keeps its bits.  Relative error (2-norm, against 64 bits, before the rounding
+// to BF16 that follows both, up to 2^-9 = 2e-3): 7.9e-8 on [-3, 0], where the
+// form above cancels (1.8e-7), 4.8e-8 on [0, 3] (3.5e-8); the network's outputs
+// are as far from 64 bits with either.
+__device__ __forceinline__ float GeluFast(float x)
 {
     const float k0 = 0.7978845608028654f, k1 = 0.044715f, c = -2.0f * 1.4426950408889634f * k0;
     float e;
@@ -623,7 +634,7 @@ __device__ __forceinline__ void HiddenEpilogue(uint32_t tbase, const float* __re
             {
                 const float2 b = __ldg(reinterpret_cast<const float2*>(bias + c0 + q * 8 + 2 * j));
                 const float z0 = v[q * 8 + 2 * j] + b.x, z1 = v[q * 8 + 2 * j + 1] + b.y;
-                p[j] = Pack2(__float2bfloat16_rn(GeluTanh(z0)), __float2bfloat16_rn(GeluTanh(z1)));
+                p[j] = Pack2(__float2bfloat16_rn(GeluFast(z0)), __float2bfloat16_rn(GeluFast(z1)));
             }
             *reinterpret_cast<uint4*>(a + CoreOffset(r, c0 / 8 + q, kHidden)) = make_uint4(p[0], p[1], p[2], p[3]);
         }

@@ -102,6 +102,22 @@ def test_fused_proposal_equals_the_three_steps():
 
 
 @pytest.mark.gpu
+def test_training_bits_are_pinned():
+    """A training run of given seeds gives the same network bit for bit, from
+    build to build: the digest of the parameters after eight steps."""
+    import hashlib
+    from hw_b200 import learned_init as L
+    net = L.Network(max_batch=256, seed=11)
+    rng = np.random.default_rng(4)
+    f = _dev(rng.standard_normal((1024, R.FEAT)).astype(np.float32))
+    t = _dev(rng.standard_normal((1024, R.OUT)).astype(np.float32))
+    net.train(f, t, epochs=2, batch=256, seed=3)
+    p, _ = net.get()
+    assert hashlib.sha256(p.tobytes()).hexdigest() == \
+        "bcab95da6f6dd0452d3cf42b286b0898d4225436f2c7eb1ddc3425e08f5262aa"
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("step", range(9))
 def test_forward_gives_up_at_every_wait_and_recovers(step):
     """Each weight copy and each commit of a tile left out in turn (a test
