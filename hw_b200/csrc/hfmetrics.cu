@@ -181,9 +181,14 @@ __device__ void HfStep(HfLane& S, const HfIn& A, int z)
             const hw_pulse p = next;
             if (bi + 1 < n) next = row[bi + 1];
             const int lb = p.label;
+            // N and NONE have no row: such a pulse counts its frames only
+            const bool base = lb < kAnalogs;
             pulseFrames += p.width;
-            ++count[kPulses][lb][z];
-            real[kMax][lb][z] = fmax_std(real[kMax][lb][z], mul_rn((float)p.max_signal, 0.1f));
+            if (base)
+            {
+                ++count[kPulses][lb][z];
+                real[kMax][lb][z] = fmax_std(real[kMax][lb][z], mul_rn((float)p.max_signal, 0.1f));
+            }
             if (pp.label != kNoneLabel)
             {
                 if (pp.label == lb) ++stutters;
@@ -198,9 +203,9 @@ __device__ void HfStep(HfLane& S, const HfIn& A, int z)
             if (!p.is_reject)
             {
                 baseFrames += p.width;
-                ++count[kBases][lb][z];
+                if (base) ++count[kBases][lb][z];
                 const float mid = MidSignal(p);
-                if (!isnan(mid))
+                if (base & !isnan(mid))
                 {
                     const uint16_t midWidth = (uint16_t)(p.width - 2);
                     ++count[kMidBases][lb][z];

@@ -170,6 +170,56 @@ def test_gpu_filter_matches_oracle_on_reference_case():
     assert _equal_metrics(got, want) is None, _equal_metrics(got, want)
 
 
+def _gpu_block(batches):
+    """The CUDA filter's metrics of one block of (pulses, lens) batches."""
+    import torch
+    from hw_b200 import filters as Fl
+    bs, models, viterbi, pd = sim_inputs()
+    hf = Fl.HfMetrics(LANES, BLOCK, 100.0, True, cart=cart())
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a).view(np.uint8).reshape(-1).copy()).cuda()
+    rest = dev(bs), dev(models), torch.from_numpy(viterbi).cuda(), dev(pd)
+    for b, (p, lens) in enumerate(batches):
+        got = hf.process(dev(p), torch.from_numpy(lens.view(np.int32)).cuda(), CAP, *rest, b * F, F)
+    return Fl.struct_to_numpy(got, abi.BASECALLING_METRICS_DT)
+
+
+def _oracle_block(batches):
+    import oracle
+    bs, models, viterbi, pd = sim_inputs()
+    ref = oracle.HfMetrics(LANES, BLOCK, 100.0, True)
+    ref.set_cart(cart())
+    for b, (p, lens) in enumerate(batches):
+        want = ref.process(p, lens, bs, models, viterbi, pd, b * F, F)
+    return want
+
+
+@pytest.mark.gpu
+def test_gpu_pulses_without_an_analog_count_their_frames_only():
+    """A pulse labelled N or NONE has no analog: it adds its frames and leaves
+    every per-analog figure as the other pulses make it."""
+    rng = np.random.default_rng(23)
+    with_n, without = [], []
+    extra = np.zeros((LANES, abi.LANE), np.int64)
+    for b in range(BLOCK // F):
+        p, lens = sim_pulses(b, n=30)
+        p["label"][:, :, :30] = rng.integers(0, 6, p["label"][:, :, :30].shape)
+        q, ql = p.copy(), np.zeros_like(lens)
+        for l in range(LANES):
+            for z in range(abi.LANE):
+                keep = p[l, z, :30][p["label"][l, z, :30] < 4]
+                ql[l, z] = len(keep)
+                q[l, z, :len(keep)] = keep
+        extra += 4 * (30 - ql.astype(np.int64))
+        with_n.append((p, lens))
+        without.append((q, ql))
+    got, want = _gpu_block(with_n), _oracle_block(without)
+    for k in ("num_pulses_by_analog", "num_bases_by_analog", "num_pk_mid_bases_by_analog", "num_pk_mid_frames",
+              "pk_mid_signal", "pk_max", "bp_zvar", "pk_zvar", "num_pulses", "num_bases"):
+        assert np.array_equal(got[k], want[k], equal_nan=got[k].dtype.kind == "f"), k
+    for k in ("num_pulse_frames", "num_base_frames"):
+        assert np.array_equal(got[k].astype(np.int64), want[k].astype(np.int64) + extra), k
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", [abi.DYNAMIC_ESTIMATIONS, abi.FIXED_ESTIMATIONS])
 def test_gpu_filter_matches_oracle_on_chain_output(mode):
