@@ -194,6 +194,20 @@ def _oracle_block(batches):
 
 
 @pytest.mark.gpu
+def test_gpu_counters_wrap_as_sixteen_bits():
+    """Pulses of up to 65,535 frames: the frame sums wrap, several times over
+    within one batch, as the reference's 16-bit counters do."""
+    rng = np.random.default_rng(17)
+    batches = [sim_pulses(b, n=CAP) for b in range(BLOCK // F)]
+    for p, _ in batches:
+        p["width"] = rng.choice(np.array([0, 1, 2, 3, 40000, 65534, 65535]), p.shape)
+        p["is_reject"] = rng.random(p.shape) < 0.3
+        p["label"] = rng.integers(0, 4, p.shape)
+    got, want = _gpu_block(batches), _oracle_block(batches)
+    assert _equal_metrics(got, want) is None, _equal_metrics(got, want)
+
+
+@pytest.mark.gpu
 def test_gpu_pulses_without_an_analog_count_their_frames_only():
     """A pulse labelled N or NONE has no analog: it adds its frames and leaves
     every per-analog figure as the other pulses make it."""
