@@ -263,16 +263,17 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
         // quotient is formed with the reciprocal of the bin size: two
         // corrections by the exact remainder (Markstein) give the IEEE
         // quotient when the reciprocal is correctly rounded and nothing
-        // under- or overflows, which `plainDiv` ensures (a quotient whose
-        // remainder underflows is far below 1 and keeps its sign).  A
-        // division instead is twice the instructions and a branch a frame,
+        // under- or overflows, which `plainDiv` ensures: a difference to the
+        // lower bound is 0 or above 2^-41, so the remainders are multiples of
+        // 2^-88.  A division instead is twice the instructions and a branch a frame,
         // which kept the frames' chains from overlapping (reset, 8 chunks of
         // 2048 lanes x 512 frames and read-out: 1490 -> 1300 us).  Chunks
-        // whose frames fill no whole batches, bin sizes out of range and a
-        // classifier without two frames of history take the division.
+        // whose frames fill no whole batches, bounds and bin sizes out of range
+        // and a classifier without two frames of history take the division.
         const float rcpBin = 1.0f / binSize;
         const bool plainDiv = binSize > 9.094947017729282e-13f && binSize < 1.099511627776e12f &&
-                              fabsf(lower) < 1.099511627776e12f;          // 2^-40, 2^40
+                              fabsf(lower) < 1.099511627776e12f &&        // 2^-40, 2^40
+                              (lower == 0.0f || fabsf(lower) > 9.094947017729282e-13f);
         auto fast = [&](const int16_t (&xA)[kHistPairBatch], const int16_t (&xB)[kHistPairBatch]) {
             float v[2][kHistPairBatch];
             bool sel[2][kHistPairBatch];

@@ -86,3 +86,30 @@ def test_histogram_edges_bit_exact():
     # the quotient-above-2^31 class was reached: those ZMWs counted low outliers
     low = want["outlier_count_low"].reshape(-1)
     assert low[1::4].sum() > 0 and want["outlier_count_high"].reshape(-1)[0::4].sum() > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lower", [4e-45, -1e-44, 1e-39, -1e-30, 1e-13, -1e-12, 0.0])
+def test_tiny_lower_bounds(lower):
+    """A difference of a value and a bound near 0 may be subnormal: its
+    quotient keeps the sign the division gives it (frames of value 0 lie in
+    bin 0 or below it)."""
+    import torch
+    from hw_b200 import filters as Fl
+    import oracle
+    cfg = workloads.small_config()
+    lanes, frames = 4, 512
+    bounds = np.zeros(lanes, abi.HIST_BOUNDS_DT)
+    bounds["lower_bounds"] = np.float32(lower)
+    bounds["upper_bounds"] = np.linspace(150.0, 1800.0, lanes * LANE).astype(np.float32).reshape(lanes, LANE)
+    models, tr = _models(lanes), np.zeros((lanes, frames, LANE), np.int16)
+    ref = oracle.Pool(cfg, lanes, frames, 0)
+    ref.hist_reset_from_bounds(bounds)
+    ref.hist_add(tr, (0, frames), models)
+    gpu = Fl.TraceHistogramAccumulator(cfg, 0, lanes)
+    gpu.reset_from_bounds(Fl.numpy_to_struct(bounds))
+    gpu.add_batch(torch.from_numpy(tr).cuda(), (0, frames), Fl.numpy_to_struct(models))
+    want, _ = ref.hist_get()
+    got = Fl.struct_to_numpy(gpu.histogram()[0], abi.LANE_HIST_DT)
+    for k in ("bin_count", "outlier_count_low", "outlier_count_high"):
+        assert np.array_equal(got[k], want[k]), k
