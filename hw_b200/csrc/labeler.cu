@@ -496,7 +496,7 @@ __device__ __forceinline__ void GroupedBackStep(uint32_t w, const float (&p)[kSt
 // differs is below 2^-102), and zero for zero; only smaller x can differ, and
 // the ROI never divides one (its dividends are 0 or sums of int16 trace values
 // times an inverse sigma of at least 1/256, so their magnitude is 0 or above
-// 2^-33).  A zero's sign may change, which no threshold sees.
+// 2^-33).
 __device__ __forceinline__ float DivByConst(float x, float c, float rcp)
 {
     const float q = mul_rn(x, rcp);
@@ -570,9 +570,12 @@ __global__ void __launch_bounds__(Threads, LabelerMinBlocks(Threads)) LabelerKer
         float p1 = mul_rn((float)pl[0], inv1);
         float p2 = mul_rn((float)pl[kLane], inv1);
         uint32_t prevRoi = (uint16_t)A.latRoi[g] & 1u;
-        // a baseline variance of 0, infinity or NaN (or a NaN threshold):
-        // comparisons instead of signs, with the reference's maxima
-        const bool plain = isfinite(inv1) & isfinite(inv2) & !isnan(k.roiUpper) & !isnan(k.roiLower);
+        // a baseline variance of 0, infinity (every statistic is then 0 or
+        // -0, whose difference to a threshold of 0 has either sign) or NaN, or
+        // a NaN threshold: comparisons instead of signs, with the reference's
+        // maxima
+        const bool plain = isfinite(inv1) & isfinite(inv2) & (inv1 > 0.0f) & (inv2 > 0.0f) & !isnan(k.roiUpper) &
+                           !isnan(k.roiLower);
         // complements of the bits, most recent frame in bit 0
         uint32_t nu = prevRoi ? 1u : 3u, nl = 0u;
         auto process = [&](float sn) {

@@ -131,6 +131,26 @@ def test_label_paths(kind, F):
     _both(cfg, lanes, F, call)
 
 
+@pytest.mark.parametrize("upper,lower", [(2.0, 0.0), (0.0, 0.0), (0.0, -0.0), (-0.0, 0.0), (0.0, 2.0)])
+def test_label_zero_threshold(upper, lower):
+    """ROI thresholds of 0 and an infinite baseline variance: the statistic is
+    0 for a positive trace and -0 for a negative one, and both reach 0."""
+    lanes, F = 2, 96
+    cfg = workloads.small_config()
+    cfg.roi_upper_threshold, cfg.roi_lower_threshold = upper, lower
+    good, bad = _models(lanes), _models(lanes)
+    bad["baseline"]["vars"][:, ::2] = 0x7c00
+    tr = synth.traces(lanes, 6 * F, seed=1, gain_sigma=0.2, empty_fraction=0.1, baseline=0.0)
+    tr[:, ::7] = 0
+
+    def call(b):
+        out = []
+        for c in range(6):
+            out += b.label(np.ascontiguousarray(tr[:, c * F:(c + 1) * F]), good if c % 2 else bad)
+        return out
+    _both(cfg, lanes, F, call)
+
+
 @pytest.mark.parametrize("kind", ["zero_var", "zero_analog_var", "nan_var", "nan_mean", "inf_var"])
 @pytest.mark.parametrize("F", [48, 512])
 def test_label_model_recovers(kind, F):
