@@ -435,13 +435,13 @@ __global__ void __launch_bounds__(kBlPairs, 16) BaselinerKernel(BaselinerArgs a,
     const int nZmw = a.lanes * kLane;
     const int nPair = nZmw / 2;
     const int gp = lane * kBlPairs + t;       // pair index; ZMWs 2 gp, 2 gp + 1
-    const int g = 2 * gp;
     const int z = 2 * t;
     const PoolStep* ps = map.On() ? &map.Pool(lane) : nullptr;
     const int F = ps ? ps->F : a.F;
 
-    // Window state: narrow windows in shared memory (one column per thread),
-    // wide ones used in place in global memory.
+    // Window state: the scales that run more often than every 16 frames in
+    // shared memory (one column per thread), the last one's used in place in
+    // global memory.
     extern __shared__ uint32_t blSmem2[];
     constexpr int NG = Lay::NumGlobalStages() > 0 ? Lay::NumGlobalStages() : 1;
     uint32_t sNext[NG];

@@ -540,8 +540,10 @@ __device__ __noinline__ void EmEStepGeneric(EmStepIo& io)
 // a ZMW, modes 0/1 and 2/3 as packed pairs.  A 4096-lane estimate took 18.5 ms
 // with the general form alone (84,900 thread instructions a ZMW and iteration)
 // and takes 10.8 ms (41,000); 37 lanes 3.35 -> 1.50 ms.  8 blocks a SM, where
-// nothing spills: before the M-step's last change 11.5 ms, 10 blocks with
-// spills 12.3 ms, 7 blocks 11.5 ms.
+// the plain estimate does not spill (the learned start's spills 24 bytes, 44
+// with the lane list, and takes 8.9 ms where the plain one takes 9.7 on the
+// same inputs): before the M-step's last change 11.5 ms, 10 blocks with spills
+// 12.3 ms, 7 blocks 11.5 ms.
 template <bool kFull = true>
 __device__ __forceinline__ float EmEStep(const KParams& k, const EmHist& h, const EmVars& v, const EmReg& r,
                                          float* bpS, float* tau0S, float* facS, float ci[5], float mom1[5],
@@ -1163,6 +1165,8 @@ __device__ __forceinline__ float EmStep(const EmVars& a, const EmVars& b)
     return d;
 }
 
+// 8 blocks a SM, where nothing spills: 20 iterations of 1024 lanes take 3.16 ms
+// (10 blocks 3.57, 12 blocks 3.91), of 37 lanes 1.49 ms (1.81, 2.06).
 __global__ void __launch_bounds__(kLane, 8) DmeEmFitKernel(DmeFitArgs A, KParams k)
 {
     const int l = blockIdx.x;

@@ -166,8 +166,9 @@ __device__ __forceinline__ float I16ToFloat(int16_t x) { return __int_as_float(0
 // next loads need sooner than their own distance can hide.
 __device__ __forceinline__ void PrefetchL1(const void* p) { asm volatile("prefetch.global.L1 [%0];" :: "l"(p)); }
 
-// Three-input maximum / minimum (one instruction on sm_100) for operands that
-// are never NaN and where the sign of a zero result does not matter.
+// Three-input maximum / minimum (one instruction on sm_100) where the sign of
+// a zero result does not matter.  A NaN operand loses to a number; the result
+// is NaN when all three are.
 __device__ __forceinline__ float max3(float a, float b, float c)
 {
     float r;
@@ -302,8 +303,6 @@ struct KParams
     // -0.0f, read at run time by the packed products (mulz2)
     float negZero;
     // labeler, 9-way rows 0, 5, 6, 7, 8: source groups 5..8 (A) and 9..12 (B);
-    // whether every such row's constants are equal within each group (then
-    // the rows take the grouped arg-max)
     // whether every such row's constants are equal within each group and every
     // constant is finite (then the labeler takes the grouped step); the
     // grouped step's constants follow, as the pairs it adds: the baseline

@@ -526,7 +526,10 @@ __device__ __noinline__ float RoiValueGeneral(float p1, float s2, float s3, floa
 
 constexpr int kBatch = 8;                              // frames loaded ahead
 
-// Blocks per SM the labeler variants are compiled for (96 registers a thread).
+// Blocks per SM the labeler variants are compiled for (96 registers a thread:
+// the grouped step spills 4 bytes in the single-pool kernel, 48 in the mapped
+// one, 28 in the mapped one with the pulses; GroupedStep has
+// the times of other block counts).
 constexpr int LabelerMinBlocks(int threads) { return threads == 64 ? 10 : threads == 128 ? 5 : 2; }
 
 // Mapped: lane-list launch.  Fuse: the pulse accumulator runs in the same

@@ -250,8 +250,6 @@ __global__ void MetricInitKernel(MetricSide S)
     for (uint32_t w = 0; w < S.lookback; ++w) S.ring[(size_t)w * S.numZmw + z] = EmptyMetricBlk();
 }
 
-// AddZmw of every ZMW z with z % stride == 0 (PrelimHQFilter.cpp:107-118,
-// MetricBufferManager.h:142-149): hq = HQ before this block's end.
 constexpr int kMetricThreads = 256;
 
 // A warp copies 32 records as consecutive words: a record a thread would touch
@@ -268,8 +266,10 @@ __device__ __forceinline__ void CopyRecords(hw_spider_metric_block* dst, const h
     for (int i = 0; i < kWords; ++i) d[i * 32 + lane] = s[i * 32 + lane];
 }
 
-__global__ void __launch_bounds__(kMetricThreads) MetricAddKernel(MetricSide S, const hw_basecalling_metrics* __restrict__ hf, const uint8_t* hq,
-                                uint32_t block)
+// AddZmw of every ZMW z with z % stride == 0 (PrelimHQFilter.cpp:107-118,
+// MetricBufferManager.h:142-149): hq = HQ before this block's end.
+__global__ void __launch_bounds__(kMetricThreads)
+MetricAddKernel(MetricSide S, const hw_basecalling_metrics* __restrict__ hf, const uint8_t* hq, uint32_t block)
 {
     const uint32_t z = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t warpZ = z & ~31u;

@@ -11,8 +11,8 @@
 
 namespace hwk {
 
-// v is 0 or at least 2^-17 (a sum of int16 values over a width): v / .1f, with
-// 10 the correctly rounded reciprocal of .1f.
+// v is 0 or at least 2^-31 (a whole number over a width): v / .1f, with 10 the
+// correctly rounded reciprocal of .1f.
 __device__ __forceinline__ uint16_t ToFixed(float v)
 {
     return static_cast<uint16_t>(add_rn(DivRcp(v, .1f, 10.0f), 0.5f));

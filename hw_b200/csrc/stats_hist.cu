@@ -338,9 +338,9 @@ HistAddKernel(hw_lane_histogram* hist, EdgeState es, const int16_t* traces, int 
         }
         int i = 0;
         // Lines of both halves some batches ahead, one a thread (a frame of
-        // the lane is one line; the first 16 are loading already): a batch
-        // ahead in registers does not cover DRAM at 10 warps a SM (1300 ->
-        // 1200 us on the case above).
+        // the lane is one line), from frame 16 of each half on; the earlier
+        // ones come with the first loads.  A batch ahead in registers does not
+        // cover DRAM at 10 warps a SM (1300 -> 1200 us on the case above).
         const int16_t* lines = tr - z + (size_t)((threadIdx.x & 16) ? S : 0) * kLane;
         const int ahead = (int)(threadIdx.x & 15);
 #pragma unroll 1
