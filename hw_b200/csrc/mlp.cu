@@ -309,11 +309,12 @@ __global__ void __launch_bounds__(128) GemmKernel(const TA* __restrict__ A, long
 // the copies and products it has in flight, writes NaN rows (a proposal the
 // DME's fallback test rejects), sets *err and returns.
 //
-// Bound by the scalar work of a tile (features, standardisation, GELU): one CTA
-// a SM by shared memory, the products a few us of the tile.  262,144 rows from
-// the histograms: 973 us with weights staged by the threads, a division and a
-// square root for every input and tanhf; 420 us with counts loaded twice, for
-// the total and for the features; 380 us as written (209 TFLOP/s).
+// Bound by latency: staging, products and epilogues of a tile run in turn, with
+// one CTA a SM by shared memory (issue 35%, XU pipe 31%, tensor pipe 8% on full
+// histograms).  262,144 rows from the histograms: 973 us with weights staged by
+// the threads, a division and a square root for every input and tanhf; 420 us
+// with counts loaded twice, for the total and for the features; 380 us as
+// written (209 TFLOP/s).
 constexpr int kTcRows = 128;
 constexpr int kTcThreads = 512;        // 16 warps: warp w reads TMEM lanes 32 (w % 4) .. + 31
 constexpr uint32_t kTcCols = 256;                                      // TMEM columns
